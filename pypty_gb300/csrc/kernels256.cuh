@@ -9,58 +9,53 @@
 
 namespace pty {
 
-// element-pair (16-byte) helpers on one block's native part: no whole-window temporaries,
-// so the window stays the only large register array
-__device__ __forceinline__ void st_native128_conj(float2* base, const float2 (&v)[32]) {
-  float4* p = reinterpret_cast<float4*>(base);
-  const int t = threadIdx.x;
+// 16-byte word helpers on one block's native part: no whole-window temporaries, so the window
+// stays the only large register array
+__device__ __forceinline__ void st_native128_conj(float2* base, const Win& v) {
+  float4* p = reinterpret_cast<float4*>(base) + nword(0, threadIdx.x);
 #pragma unroll
-  for (int j = 0; j < 16; ++j) p[j * 512 + t] = make_float4(v[2 * j].x, -v[2 * j].y, v[2 * j + 1].x, -v[2 * j + 1].y);
+  for (int j = 0; j < 16; ++j) p[j * 32] = pack4(v.re[j], pneg(v.im[j]));
 }
 
 // v *= w (conj_w: v *= conj(w)) for w in native order at base
-__device__ __forceinline__ void mul_native128(float2 (&v)[32], const float2* base, bool conj_w) {
-  const float4* p = reinterpret_cast<const float4*>(base);
-  const int t = threadIdx.x;
+__device__ __forceinline__ void mul_native128(Win& v, const float2* base, bool conj_w) {
+  const float4* p = reinterpret_cast<const float4*>(base) + nword(0, threadIdx.x);
 #pragma unroll
   for (int j = 0; j < 16; ++j) {
-    const float4 q = p[j * 512 + t];
-    const float2 w0 = make_float2(q.x, q.y), w1 = make_float2(q.z, q.w);
-    v[2 * j] = conj_w ? cmulc(v[2 * j], w0) : cmul(v[2 * j], w0);
-    v[2 * j + 1] = conj_w ? cmulc(v[2 * j + 1], w1) : cmul(v[2 * j + 1], w1);
+    const float4 q = p[j * 32];
+    const float2 wi = make_float2(q.z, q.w), ni = pneg(wi);
+    pcmul(v.re[j], v.im[j], make_float2(q.x, q.y), conj_w ? ni : wi, conj_w ? wi : ni);
     if ((j & 7) == 7) asm volatile("" ::: "memory");
   }
 }
 
 // out = (accumulate ? out : 0) + a * v with a, out in native order
-__device__ __forceinline__ void madd_native128(float2* out, const float2* a_, const float2 (&v)[32], bool accumulate) {
-  float4* o = reinterpret_cast<float4*>(out);
-  const float4* a = reinterpret_cast<const float4*>(a_);
-  const int t = threadIdx.x;
+__device__ __forceinline__ void madd_native128(float2* out, const float2* a_, const Win& v, bool accumulate) {
+  float4* o = reinterpret_cast<float4*>(out) + nword(0, threadIdx.x);
+  const float4* a = reinterpret_cast<const float4*>(a_) + nword(0, threadIdx.x);
 #pragma unroll
   for (int j = 0; j < 16; ++j) {
-    const float4 q = a[j * 512 + t];
-    float2 g0 = cmul(make_float2(q.x, q.y), v[2 * j]);
-    float2 g1 = cmul(make_float2(q.z, q.w), v[2 * j + 1]);
+    const float4 q = a[j * 32];
+    float2 gr = make_float2(q.x, q.y), gi = make_float2(q.z, q.w);
+    pcmul(gr, gi, v.re[j], v.im[j], pneg(v.im[j]));
     if (accumulate) {
-      const float4 r = o[j * 512 + t];
-      g0 = cadd(make_float2(r.x, r.y), g0);
-      g1 = cadd(make_float2(r.z, r.w), g1);
+      const float4 r = o[j * 32];
+      gr = padd(make_float2(r.x, r.y), gr);
+      gi = padd(make_float2(r.z, r.w), gi);
     }
-    o[j * 512 + t] = make_float4(g0.x, g0.y, g1.x, g1.y);
+    o[j * 32] = pack4(gr, gi);
     if ((j & 3) == 3) asm volatile("" ::: "memory");   // bound the loads in flight
   }
 }
 
 // v += w (native order)
-__device__ __forceinline__ void add_native128(float2 (&v)[32], const float2* base) {
-  const float4* p = reinterpret_cast<const float4*>(base);
-  const int t = threadIdx.x;
+__device__ __forceinline__ void add_native128(Win& v, const float2* base) {
+  const float4* p = reinterpret_cast<const float4*>(base) + nword(0, threadIdx.x);
 #pragma unroll
   for (int j = 0; j < 16; ++j) {
-    const float4 q = p[j * 512 + t];
-    v[2 * j] = cadd(v[2 * j], make_float2(q.x, q.y));
-    v[2 * j + 1] = cadd(v[2 * j + 1], make_float2(q.z, q.w));
+    const float4 q = p[j * 32];
+    v.re[j] = padd(v.re[j], make_float2(q.x, q.y));
+    v.im[j] = padd(v.im[j], make_float2(q.z, q.w));
   }
 }
 
@@ -70,11 +65,11 @@ struct Smem256 {
   static constexpr size_t xbuf_off = 0;
   static constexpr size_t tw1_off = xbuf_off + sizeof(float2) * G::XBUF;
   static constexpr size_t tw2_off = tw1_off + sizeof(float2) * G::TW1;
-  static constexpr size_t tw256_off = tw2_off + sizeof(float2) * G::TW2;
+  static constexpr size_t tw256_off = tw2_off + sizeof(float2) * 2 * G::TW2;
   static constexpr size_t red_off = tw256_off + sizeof(float2) * 256;
   static constexpr size_t small = red_off + sizeof(double) * 72;              // FFT-only kernels
   static constexpr size_t pyx_off = small;
-  static constexpr size_t bits_off = pyx_off + sizeof(float2) * 512;
+  static constexpr size_t bits_off = pyx_off + sizeof(float2) * 3 * 256;   // y factors as packs, x factors
   static constexpr size_t acc_off = bits_off + sizeof(uint32_t) * G::T * 4;
   static constexpr size_t fused = acc_off + sizeof(float) * G::XBUF;         // the fused kernel
 };
@@ -104,11 +99,11 @@ __global__ void __launch_bounds__(512, 1) probe_fft256_kernel(const float2* __re
   load_twiddles<128>(s.tw1, s.tw2, g_tw);
   load_tw256(s.tw256);
   __syncthreads();
-  float2 v[32];
+  Win v;
 #pragma unroll
-  for (int i = 0; i < 32; ++i) v[i] = probe[(size_t)(G::ry(c, t) * 256 + G::rx(c, t, i)) * Mp + p];
+  for (int i = 0; i < 32; ++i) wset(v, i, probe[(size_t)(G::ry(c, t) * 256 + G::rx(c, t, i)) * Mp + p]);
   WinFFT256::forward(v, s.xbuf, s.tw1, s.tw2, s.tw256, cl);
-  st_native<128>(probe_f + (size_t)p * 65536 + c * G::PART, v);
+  st_native(probe_f + (size_t)p * 65536 + c * G::PART, v);
 }
 
 // ------------------------------------------------------------------ object windows
@@ -125,12 +120,12 @@ __global__ void __launch_bounds__(512, 1) object_windows256_kernel(WindowArgs a)
   const int gi = a.seq[b];
   const int y0 = a.pos[2 * gi], x0 = a.pos[2 * gi + 1];
   const float2* src = a.obj + (size_t)k * a.Ny * a.Nx + (size_t)(y0 + G::ry(c, t)) * a.Nx + x0;
-  float2 v[32];
+  Win v;
 #pragma unroll
-  for (int i = 0; i < 32; ++i) v[i] = src[G::rx(c, t, i)];
+  for (int i = 0; i < 32; ++i) wset(v, i, src[G::rx(c, t, i)]);
   __syncthreads();
   WinFFT256::band_limit(v, s.xbuf, s.tw1, s.tw2, s.tw256, cl, a.mask_sc);
-  st_native<128>(a.out + (size_t)win * 65536 + c * G::PART, v);
+  st_native(a.out + (size_t)win * 65536 + c * G::PART, v);
 }
 
 // ------------------------------------------------------------------ gradient windows
@@ -145,13 +140,13 @@ __global__ void __launch_bounds__(512, 1) grad_windows256_kernel(float2* buf, co
   float2* win = buf + (size_t)(blockIdx.x / 4) * 65536;
   load_twiddles<128>(s.tw1, s.tw2, g_tw);
   load_tw256(s.tw256);
-  float2 v[32];
-  ld_native<128>(win + c * G::PART, v);
+  Win v;
+  ld_native(win + c * G::PART, v);
   __syncthreads();
   // the cluster barriers inside the transforms order every block's reads before any write
   WinFFT256::band_limit(v, s.xbuf, s.tw1, s.tw2, s.tw256, cl, mask_sc);
 #pragma unroll
-  for (int i = 0; i < 32; ++i) win[G::ry(c, t) * 256 + G::rx(c, t, i)] = v[i];
+  for (int i = 0; i < 32; ++i) win[G::ry(c, t) * 256 + G::rx(c, t, i)] = wget(v, i);
 }
 
 // ------------------------------------------------------------------ probe gradient
@@ -167,21 +162,22 @@ __global__ void __launch_bounds__(512, 1) probe_final256_kernel(const float2* __
   load_twiddles<128>(s.tw1, s.tw2, g_tw);
   load_tw256(s.tw256);
   __syncthreads();
-  // chunks outer, elements inner: each chunk's 32 loads are in flight together (the chunk
-  // order of every element's sum is unchanged)
-  float2 v[32];
+  // chunks outer, elements inner: each chunk's loads are in flight together (the chunk order of
+  // every element's sum is unchanged)
+  Win v;
 #pragma unroll
-  for (int i = 0; i < 32; ++i) v[i] = make_float2(0.f, 0.f);
-  for (int ch = 0; ch < nchunk; ++ch) {
-    const float2* src = partial + ((size_t)ch * Mp + p) * 65536 + c * G::PART;
+  for (int j = 0; j < 16; ++j) v.re[j] = v.im[j] = make_float2(0.f, 0.f);
+  for (int ch = 0; ch < nchunk; ++ch) add_native128(v, partial + ((size_t)ch * Mp + p) * 65536 + c * G::PART);
 #pragma unroll
-    for (int i = 0; i < 32; ++i) v[i] = cadd(v[i], src[nidx<128>(i, t)]);
+  for (int j = 0; j < 16; ++j) {
+    const float* m = mask_sc + G::fky(c, t, 2 * j) * 256 + G::fkx(c, t, 2 * j);
+    const float2 mk = make_float2(m[0], m[64]);
+    v.re[j] = pmul(v.re[j], mk);
+    v.im[j] = pmul(v.im[j], mk);
   }
-#pragma unroll
-  for (int i = 0; i < 32; ++i) v[i] = cscale(v[i], mask_sc[G::fky(c, t, i) * 256 + G::fkx(c, t, i)]);
   WinFFT256::inverse(v, s.xbuf, s.tw1, s.tw2, s.tw256, cl);
 #pragma unroll
-  for (int i = 0; i < 32; ++i) probe_grad[(size_t)(G::ry(c, t) * 256 + G::rx(c, t, i)) * Mp + p] = v[i];
+  for (int i = 0; i < 32; ++i) probe_grad[(size_t)(G::ry(c, t) * 256 + G::rx(c, t, i)) * Mp + p] = wget(v, i);
 }
 
 // ------------------------------------------------------------------ plain batched FFT
@@ -198,22 +194,22 @@ __global__ void __launch_bounds__(512, 1) fft2_batch256_kernel(const float2* __r
   const float2* src = in + (size_t)(blockIdx.x / 4) * 65536;
   float2* dst = out + (size_t)(blockIdx.x / 4) * 65536;
   const int h = shift ? 128 : 0;
-  float2 v[32];
+  Win v;
   if (!inverse) {
 #pragma unroll
-    for (int i = 0; i < 32; ++i) v[i] = src[G::ry(c, t) * 256 + G::rx(c, t, i)];
+    for (int i = 0; i < 32; ++i) wset(v, i, src[G::ry(c, t) * 256 + G::rx(c, t, i)]);
     WinFFT256::forward(v, s.xbuf, s.tw1, s.tw2, s.tw256, cl);
 #pragma unroll
     for (int i = 0; i < 32; ++i)
-      dst[((G::fky(c, t, i) + h) & 255) * 256 + ((G::fkx(c, t, i) + h) & 255)] = v[i];
+      dst[((G::fky(c, t, i) + h) & 255) * 256 + ((G::fkx(c, t, i) + h) & 255)] = wget(v, i);
   } else {
     const float inv = 1.0f / 65536.0f;
 #pragma unroll
     for (int i = 0; i < 32; ++i)
-      v[i] = cscale(src[((G::fky(c, t, i) + h) & 255) * 256 + ((G::fkx(c, t, i) + h) & 255)], inv);
+      wset(v, i, cscale(src[((G::fky(c, t, i) + h) & 255) * 256 + ((G::fkx(c, t, i) + h) & 255)], inv));
     WinFFT256::inverse(v, s.xbuf, s.tw1, s.tw2, s.tw256, cl);
 #pragma unroll
-    for (int i = 0; i < 32; ++i) dst[G::ry(c, t) * 256 + G::rx(c, t, i)] = v[i];
+    for (int i = 0; i < 32; ++i) dst[G::ry(c, t) * 256 + G::rx(c, t, i)] = wget(v, i);
   }
 }
 
@@ -234,9 +230,9 @@ __global__ void __launch_bounds__(512, 1) layered_step256_kernel(float2* x, cons
   float2* win = x + w * 65536;
   load_twiddles<128>(s.tw1, s.tw2, g_tw);
   load_tw256(s.tw256);
-  float2 v[32];
+  Win v;
 #pragma unroll
-  for (int i = 0; i < 32; ++i) v[i] = win[G::ry(c, t) * 256 + G::rx(c, t, i)];
+  for (int i = 0; i < 32; ++i) wset(v, i, win[G::ry(c, t) * 256 + G::rx(c, t, i)]);
   __syncthreads();
   // the cluster barriers inside the transforms order every block's reads before any write
   if (rtab)
@@ -244,7 +240,7 @@ __global__ void __launch_bounds__(512, 1) layered_step256_kernel(float2* x, cons
   else
     WinFFT256::propagate(v, s.xbuf, s.tw1, s.tw2, s.tw256, cl, tab + (w / nper) * tab_stride, conj != 0, scale);
 #pragma unroll
-  for (int i = 0; i < 32; ++i) win[G::ry(c, t) * 256 + G::rx(c, t, i)] = v[i];
+  for (int i = 0; i < 32; ++i) win[G::ry(c, t) * 256 + G::rx(c, t, i)] = wget(v, i);
 }
 
 // One forward multislice step of the layered path for 256-px windows (multislice_core.py:61-80)
@@ -268,19 +264,19 @@ __global__ void __launch_bounds__(512, 1) layered_fwd256_kernel(const float2* __
   const float2* o = ob + (((size_t)b * Z + z) * Mo + m) * WW;
   load_twiddles<128>(s.tw1, s.tw2, g_tw);
   load_tw256(s.tw256);
-  float2 v[32];
+  Win v;
 #pragma unroll
   for (int i = 0; i < 32; ++i) {
     const int u = G::ry(c, t) * 256 + G::rx(c, t, i);
     const float2 in = src[u];
     stw[u] = cconj(in);
-    v[i] = cmul(in, o[u]);
+    wset(v, i, cmul(in, o[u]));
   }
   __syncthreads();
   WinFFT256::propagate(v, s.xbuf, s.tw1, s.tw2, s.tw256, cl, tab + (size_t)b * tab_stride, false, scale);
   float2* dst = psi + (size_t)wi * WW;
 #pragma unroll
-  for (int i = 0; i < 32; ++i) dst[G::ry(c, t) * 256 + G::rx(c, t, i)] = v[i];
+  for (int i = 0; i < 32; ++i) dst[G::ry(c, t) * 256 + G::rx(c, t, i)] = wget(v, i);
 }
 
 // ------------------------------------------------------------------ fused multislice, 256
@@ -319,10 +315,10 @@ __global__ void __launch_bounds__(512, 1) fused256_kernel(FusedArgs a) {
   constexpr size_t PART = G::PART;
   extern __shared__ __align__(16) unsigned char smem[];
   Carve256 s(smem);
-  float2* spy = reinterpret_cast<float2*>(smem + Smem256::pyx_off);   // [256] y factor, [256] x factor
-  const float2* spx = spy + 256;
+  float4* spy = reinterpret_cast<float4*>(smem + Smem256::pyx_off);   // [256] y factor (re, re, im, im)
+  float2* spx = reinterpret_cast<float2*>(spy + 256);                 // [256] x factor
   uint32_t* sbits = reinterpret_cast<uint32_t*>(smem + Smem256::bits_off);
-  float* facc = reinterpret_cast<float*>(smem + Smem256::acc_off);     // I accumulator, then dL/dI
+  float2* facc = reinterpret_cast<float2*>(smem + Smem256::acc_off);   // per pack [16][T]: I accumulator, then dL/dI
   double* xch = s.red + 64;                                            // cluster exchange slots
   cg::cluster_group cl = cg::this_cluster();
   const int c = (int)cl.block_rank(), t = threadIdx.x;
@@ -333,14 +329,18 @@ __global__ void __launch_bounds__(512, 1) fused256_kernel(FusedArgs a) {
   const int nck = (Z + K - 1) / K;
   load_twiddles<128>(s.tw1, s.tw2, a.tw);
   load_tw256(s.tw256);
-  for (int i = t; i < 512; i += T) spy[i] = a.pyx[i];
+  for (int i = t; i < 256; i += T) {
+    const float2 y = a.pyx[i];
+    spy[i] = make_float4(y.x, y.x, y.y, y.y);
+    spx[i] = a.pyx[256 + i];
+  }
   for (int q = 0; q < 4; ++q) {   // band-limit bits of this thread's elements in every quadrant
     uint32_t mb = 0;
 #pragma unroll
     for (int i = 0; i < 32; ++i) mb |= (a.mask[G::fky(q, t, i) * 256 + G::fkx(q, t, i)] != 0.0f ? 1u : 0u) << i;
     sbits[q * T + t] = mb;
   }
-  for (int i = 0; i < 32; ++i) facc[i * T + t] = 0.0f;
+  for (int j = 0; j < 16; ++j) facc[j * T + t] = make_float2(0.f, 0.f);
   const bool want_probe = a.step_probe || a.step_pos;
   auto part = [&](const float2* base, size_t win) { return base + win * WW + c * PART; };
   auto wpart = [&](float2* base, size_t win) { return base + win * WW + c * PART; };
@@ -348,11 +348,12 @@ __global__ void __launch_bounds__(512, 1) fused256_kernel(FusedArgs a) {
 
   int stage = FWD ? F_START : A_START, k = 0, z = 0, z0 = 0, zl = 0;
   if (ADJ) {
-    for (int i = 0; i < 32; ++i) facc[i * T + t] = a.dldi[(size_t)b * WW + c * PART + i * T + t];
+    const float2* src = reinterpret_cast<const float2*>(a.dldi + (size_t)b * WW + c * PART);
+    for (int j = 0; j < 16; ++j) facc[j * T + t] = src[j * T + t];
   }
   __syncthreads();
 
-  float2 v[32];
+  Win v;
   while (stage != S_DONE) {
     const bool fwd_stage = FWD;
     const int p = fwd_stage ? k % Mp : k / Mo;
@@ -367,7 +368,8 @@ __global__ void __launch_bounds__(512, 1) fused256_kernel(FusedArgs a) {
       double lsum = 0.0, ssum = 0.0;
 #pragma unroll 1
       for (int i = 0; i < 32; ++i) {
-        const float acc = facc[i * T + t];
+        float& acc_ref = reinterpret_cast<float*>(facc + (i >> 1) * T + t)[i & 1];
+        const float acc = acc_ref;
         const float I = (nmodes == 1) ? acc : acc * inv_modes;
         const int ky = G::fky(c, t, i), kx = G::fkx(c, t, i);
         const int didx = ((ky + 128) & 255) * 256 + ((kx + 128) & 255);
@@ -377,7 +379,7 @@ __global__ void __launch_bounds__(512, 1) fused256_kernel(FusedArgs a) {
         }
         float d = loss_pixel(a.algorithm, I, meas[didx], lsum, ssum);
         if (nmodes > 1) d = d / (float)nmodes;
-        facc[i * T + t] = d;
+        acc_ref = d;
       }
       if (a.simulate) return;
       block_sum2(lsum, ssum, s.red);
@@ -397,7 +399,8 @@ __global__ void __launch_bounds__(512, 1) fused256_kernel(FusedArgs a) {
         a.loss_part[2 * b + 1] = q;
       }
       cl.sync();
-      for (int i = 0; i < 32; ++i) a.dldi[(size_t)b * WW + c * PART + i * T + t] = facc[i * T + t];
+      float2* dst = reinterpret_cast<float2*>(a.dldi + (size_t)b * WW + c * PART);
+      for (int j = 0; j < 16; ++j) dst[j * T + t] = facc[j * T + t];
       return;
     }
 
@@ -425,7 +428,7 @@ __global__ void __launch_bounds__(512, 1) fused256_kernel(FusedArgs a) {
     // ------------------------------------------------ real-space op
     bool do_fwd = false, do_inv = false, skip = false;
     if (FWD && stage == F_START) {
-      ld_native<128>(part(a.fprobe, (size_t)b * Mp + p), v);   // the shifted incoming probe
+      ld_native(part(a.fprobe, (size_t)b * Mp + p), v);   // the shifted incoming probe
     } else if (ADJ && stage == A_START) {
       do_inv = true;
     } else if (FWD) {   // F_SLICE
@@ -435,10 +438,10 @@ __global__ void __launch_bounds__(512, 1) fused256_kernel(FusedArgs a) {
       do_inv = z < Z - 1;
     } else if (stage == A_RECOMP) {
       if (z == z0) {
-        st_native<128>(wpart(a.gpark, b), v);                 // park the adjoint wave
-        ld_native<128>(part(a.stack, stack_win(z0, p, m)), v);
+        st_native(wpart(a.gpark, b), v);                 // park the adjoint wave
+        ld_native(part(a.stack, stack_win(z0, p, m)), v);
 #pragma unroll
-        for (int i = 0; i < 32; ++i) v[i] = cconj(v[i]);     // the checkpoint holds conj(psi)
+        for (int j = 0; j < 16; ++j) v.im[j] = pneg(v.im[j]);     // the checkpoint holds conj(psi)
       }
       st_native128_conj(wpart(a.seg, (size_t)b * K + (z - z0)), v);
       if (z < zl) {
@@ -446,7 +449,7 @@ __global__ void __launch_bounds__(512, 1) fused256_kernel(FusedArgs a) {
         do_fwd = true;
         do_inv = true;
       } else {
-        ld_native<128>(part(a.gpark, b), v);                  // the adjoint wave back
+        ld_native(part(a.gpark, b), v);                  // the adjoint wave back
       }
     } else {   // A_SLICE
       if (store_stack) {
@@ -464,12 +467,12 @@ __global__ void __launch_bounds__(512, 1) fused256_kernel(FusedArgs a) {
           float2* pr = wpart(a.pgr, (size_t)b * Mp + p);
           if (m > 0) add_native128(v, pr);
           if (m < Mo - 1) {
-            st_native<128>(pr, v);
+            st_native(pr, v);
             skip = true;
           }
         }
         // the probe-gradient wave; probe_spectrum256_kernel takes its spectrum
-        if (!skip) st_native<128>(wpart(a.fprobe, (size_t)b * Mp + p), v);
+        if (!skip) st_native(wpart(a.fprobe, (size_t)b * Mp + p), v);
       }
     }
 
@@ -489,10 +492,41 @@ __global__ void __launch_bounds__(512, 1) fused256_kernel(FusedArgs a) {
       const bool edge = a.use_edge && zstep == 0;
       const bool tab = !a.use_sep || edge;
       const float2* pr = a.prop_steps ? a.prop_steps + (size_t)zstep * (256 * 256) : (edge ? a.prop_edge : a.prop);
-      WinFFT256::cross_propagate(v, s.xbuf, cl, c, adjoint, [&](int i, int q) {
-        const int ky = G::fky(q, t, i), kx = G::fkx(q, t, i);
-        if (tab) return pr[ky * 256 + kx];
-        return ((sbits[q * T + t] >> i) & 1u) ? cmul(spy[ky], spx[kx]) : make_float2(0.f, 0.f);
+      // separable: sum over q_y of P_y (sum over q_x of P_x Z_q), Z_q zero outside the band; a
+      // thread's packs share kx, so the x factors of the two column quadrants are held
+      float2 xr[2], xi[2];
+#pragma unroll
+      for (int qx = 0; qx < 2; ++qx) {
+        const float2* x = spx + G::fkx(qx, t, 0);
+        xr[qx] = make_float2(x[0].x, x[64].x);
+        xi[qx] = adjoint ? make_float2(-x[0].y, -x[64].y) : make_float2(x[0].y, x[64].y);
+      }
+      WinFFT256::cross_propagate(v, s.xbuf, cl, c, [&](int j, float2 (&zr)[4], float2 (&zi)[4], float2& re, float2& im) {
+        if (tab) {
+          WinFFT256::mul_quadrants(t, j, zr, zi, pr, adjoint, re, im);
+          return;
+        }
+#pragma unroll
+        for (int qy = 0; qy < 2; ++qy) {
+          float2 sr, si;
+#pragma unroll
+          for (int qx = 0; qx < 2; ++qx) {
+            const int q = 2 * qy + qx;
+            const uint32_t mb = sbits[q * T + t] >> (2 * j);
+            const float2 ar = make_float2((mb & 1u) ? zr[q].x : 0.f, (mb & 2u) ? zr[q].y : 0.f);
+            const float2 ai = make_float2((mb & 1u) ? zi[q].x : 0.f, (mb & 2u) ? zi[q].y : 0.f);
+            sr = qx ? pfma(ar, xr[qx], sr) : pmul(ar, xr[qx]);
+            si = qx ? pfma(ai, xr[qx], si) : pmul(ai, xr[qx]);
+            sr = pfma(ai, pneg(xi[qx]), sr);
+            si = pfma(ar, xi[qx], si);
+          }
+          const float4 y = spy[G::fky(2 * qy, t, 2 * j)];
+          const float2 yr = make_float2(y.x, y.y), yi = adjoint ? make_float2(-y.z, -y.w) : make_float2(y.z, y.w);
+          re = qy ? pfma(sr, yr, re) : pmul(sr, yr);
+          im = qy ? pfma(si, yr, im) : pmul(si, yr);
+          re = pfma(si, pneg(yi), re);
+          im = pfma(sr, yi, im);
+        }
       });
     } else {
       // outside the propagation steps only the far field (forward) transforms forward: the
@@ -500,17 +534,24 @@ __global__ void __launch_bounds__(512, 1) fused256_kernel(FusedArgs a) {
       if (FWD && do_fwd) WinFFT256::cross(v, s.xbuf, cl, c);
       if (ADJ && stage == A_START) {
         // dL/dPsi = dL/dI * Psi * w (objective.py:595-597)
-        ld_native<128>(part(a.psi, (size_t)b * nmodes + kidx), v);
+        ld_native(part(a.psi, (size_t)b * nmodes + kidx), v);
 #pragma unroll
-        for (int i = 0; i < 32; ++i) v[i] = cscale(cscale(v[i], facc[i * T + t]), a.loss_weight);
+        for (int j = 0; j < 16; ++j) {
+          const float2 d = facc[j * T + t], lw = pdup(a.loss_weight);
+          v.re[j] = pmul(pmul(v.re[j], d), lw);
+          v.im[j] = pmul(pmul(v.im[j], d), lw);
+        }
       } else if (FWD && stage == F_SLICE && z == Z - 1) {   // the exit plane
         // far field of this mode: Psi = FFT(exit) * mask; accumulate |Psi|^2
 #pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          v[i] = cscale(v[i], a.mask[G::fky(c, t, i) * 256 + G::fkx(c, t, i)]);
-          facc[i * T + t] += cabs2(v[i]);
+        for (int j = 0; j < 16; ++j) {
+          const float* mp = a.mask + G::fky(c, t, 2 * j) * 256 + G::fkx(c, t, 2 * j);
+          const float2 mk = make_float2(mp[0], mp[64]);
+          v.re[j] = pmul(v.re[j], mk);
+          v.im[j] = pmul(v.im[j], mk);
+          facc[j * T + t] = padd(facc[j * T + t], pfma(v.im[j], v.im[j], pmul(v.re[j], v.re[j])));
         }
-        if (!a.simulate) st_native<128>(wpart(a.psi, (size_t)b * nmodes + kidx), v);
+        if (!a.simulate) st_native(wpart(a.psi, (size_t)b * nmodes + kidx), v);
       }
       if (do_inv) WinFFT256::cross(v, s.xbuf, cl, c);
     }
@@ -580,7 +621,7 @@ __global__ void __launch_bounds__(512, 1) shifted_probes256_kernel(FusedArgs a) 
   const float inv = 1.0f / (float)WW;
   const int gi = a.seq[b];
   const float dy = a.corr[2 * gi], dx = a.corr[2 * gi + 1];
-  float2 v[32];
+  Win v;
 #pragma unroll
   for (int i = 0; i < 32; ++i) {
     float2 w = make_float2(inv, 0.f);
@@ -592,10 +633,10 @@ __global__ void __launch_bounds__(512, 1) shifted_probes256_kernel(FusedArgs a) 
       sincosf(th, &sn, &cs);
       w = make_float2(cs * mk * inv, sn * mk * inv);
     }
-    v[i] = cmul(pf[nidx<128>(i, t)], w);
+    wset(v, i, cmul(native_at(pf, i, t), w));
   }
   WinFFT256::inverse(v, s.xbuf, s.tw1, s.tw2, s.tw256, cl);
-  st_native<128>(a.fprobe + (size_t)win * WW + c * G::PART, v);
+  st_native(a.fprobe + (size_t)win * WW + c * G::PART, v);
 }
 
 // ------------------------------------------------------------------ probe-gradient spectrum
@@ -614,8 +655,8 @@ __global__ void __launch_bounds__(512, 1) probe_spectrum256_kernel(FusedArgs a) 
   load_twiddles<128>(s.tw1, s.tw2, a.tw);
   load_tw256(s.tw256);
   float2* dst = a.fprobe + (size_t)win * WW + c * G::PART;
-  float2 v[32];
-  ld_native<128>(dst, v);
+  Win v;
+  ld_native(dst, v);
   __syncthreads();
   WinFFT256::forward(v, s.xbuf, s.tw1, s.tw2, s.tw256, cl);
   double gy = 0.0, gx = 0.0;
@@ -630,15 +671,16 @@ __global__ void __launch_bounds__(512, 1) probe_spectrum256_kernel(FusedArgs a) 
       const float th = __fadd_rn(__fmul_rn(__fmul_rn(a.sx[kx], mk), dx), __fmul_rn(__fmul_rn(a.sy[ky], mk), dy));
       float sn, cs;
       sincosf(th, &sn, &cs);
-      v[i] = cmulc(v[i], make_float2(cs * mk, sn * mk));
+      const float2 g = cmulc(wget(v, i), make_float2(cs * mk, sn * mk));
+      wset(v, i, g);
       if (a.step_pos) {
-        const float im = cmulc(v[i], pf[nidx<128>(i, t)]).y;
+        const float im = cmulc(g, native_at(pf, i, t)).y;
         gy += (double)(-(a.sy[ky] * mk) * im);
         gx += (double)(-(a.sx[kx] * mk) * im);
       }
     }
   }
-  if (a.step_probe) st_native<128>(dst, v);
+  if (a.step_probe) st_native(dst, v);
   if (a.step_pos) {
     block_sum2(gy, gx, s.red);
     if (t == 0) {

@@ -496,13 +496,13 @@ int run_ms_forward(const MsPlan& q, const float2* probe_b, const float2* obj_b, 
   int rc = ms_tables<W>(q, propagator, edge_mult, nullptr, ws, st);
   if (rc) return rc;
   prof_mark(st, KID_LAYOUT);
-  ref_to_native_kernel<W><<<q.B * q.Mp, T, 0, st>>>(probe_b, at<float2>(ws, q.o_probe_b), q.Mp);
-  ref_to_native_kernel<W><<<q.B * q.zm, T, 0, st>>>(obj_b, at<float2>(ws, q.o_obl), q.zm);
+  ref_to_native_kernel<W><<<q.B * q.Mp, T, 0, st>>>(probe_b, at<float2>(ws, q.o_probe_b), q.Mp, 0);
+  ref_to_native_kernel<W><<<q.B * q.zm, T, 0, st>>>(obj_b, at<float2>(ws, q.o_obl), q.zm, 0);
   if ((rc = ms_fused<W>(q, 3, 1, 0, (edge_mult > 1.0f && q.Z > 1) ? 1 : 0, ws, st))) return rc;
   prof_mark(st, KID_LAYOUT);
   native_to_ref_kernel<W><<<q.B * q.Z * q.Mp * q.Mo, T, 0, st>>>(at<float2>(ws, q.o_stack), waves,
-                                                                q.Z * q.Mp * q.Mo);
-  native_to_ref_kernel<W><<<q.B * q.Mp * q.Mo, T, 0, st>>>(at<float2>(ws, q.o_gbuf), exit_wave, q.Mp * q.Mo);
+                                                                q.Z * q.Mp * q.Mo, 1);
+  native_to_ref_kernel<W><<<q.B * q.Mp * q.Mo, T, 0, st>>>(at<float2>(ws, q.o_gbuf), exit_wave, q.Mp * q.Mo, 0);
   prof_mark(st, -1);
   return cuda_status();
 }
@@ -516,11 +516,11 @@ int run_ms_grads(const MsPlan& q, const float2* d_exit, const float2* waves, con
   int rc = ms_tables<W>(q, propagator, edge_mult, mask_clean, ws, st);
   if (rc) return rc;
   prof_mark(st, KID_LAYOUT);
-  ref_to_native_kernel<W><<<q.B * q.Mp * q.Mo, T, 0, st>>>(d_exit, at<float2>(ws, q.o_gbuf), q.Mp * q.Mo);
-  ref_to_native_kernel<W><<<q.B * q.zm, T, 0, st>>>(obj_b, at<float2>(ws, q.o_obl), q.zm);
+  ref_to_native_kernel<W><<<q.B * q.Mp * q.Mo, T, 0, st>>>(d_exit, at<float2>(ws, q.o_gbuf), q.Mp * q.Mo, 0);
+  ref_to_native_kernel<W><<<q.B * q.zm, T, 0, st>>>(obj_b, at<float2>(ws, q.o_obl), q.zm, 0);
   if (step_obj)
     ref_to_native_kernel<W><<<q.B * q.Z * q.Mp * q.Mo, T, 0, st>>>(waves, at<float2>(ws, q.o_stack),
-                                                                  q.Z * q.Mp * q.Mo);
+                                                                  q.Z * q.Mp * q.Mo, 1);
   if ((rc = ms_fused<W>(q, 4, step_obj, probe_grad != nullptr, (edge_mult > 1.0f && q.Z > 1) ? 1 : 0, ws, st)))
     return rc;
   if (step_obj) {
@@ -544,7 +544,7 @@ int run_ms_grads(const MsPlan& q, const float2* d_exit, const float2* waves, con
   }
   if (probe_grad) {
     prof_mark(st, KID_LAYOUT);
-    native_to_ref_kernel<W><<<q.B * q.Mp, T, 0, st>>>(at<float2>(ws, q.o_fprobe), probe_grad, q.Mp);
+    native_to_ref_kernel<W><<<q.B * q.Mp, T, 0, st>>>(at<float2>(ws, q.o_fprobe), probe_grad, q.Mp, 0);
   }
   (void)WW;
   prof_mark(st, -1);

@@ -1,8 +1,8 @@
 // Kernels of the far-field multislice loss-and-gradient path (pypty objective /
 // multislice_core restated for sm_103a). All kernels are templated on the window size W
 // and use WinFFT<W> for their transforms. Windows that live only inside one call are
-// stored in the "native" order of WinFFT (element i of thread t at offset i*T + t) so that
-// every load/store of a window is a fully coalesced 256-byte warp access.
+// stored in the "native" order of WinFFT (each thread's element pairs, warp by warp) so that
+// every load/store of a window is a fully coalesced 512-byte warp access.
 #pragma once
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
@@ -188,7 +188,7 @@ static __global__ void slices_to_obj_kernel(const float2* __restrict__ src, floa
 template <int W>
 struct Smem {
   using G = Geo<W>;
-  static constexpr size_t bytes = sizeof(float2) * (G::XBUF + G::TW1 + G::TW2) + sizeof(double) * 64;
+  static constexpr size_t bytes = sizeof(float2) * (G::XBUF + G::TW1 + 2 * G::TW2) + sizeof(double) * 64;
 };
 
 template <int W>
@@ -198,7 +198,7 @@ __device__ __forceinline__ void carve(unsigned char* smem, float2*& xbuf, float2
   xbuf = reinterpret_cast<float2*>(smem);
   tw1 = xbuf + G::XBUF;
   tw2 = tw1 + G::TW1;
-  red = reinterpret_cast<double*>(tw2 + G::TW2);
+  red = reinterpret_cast<double*>(tw2 + 2 * G::TW2);
 }
 
 // sum of (a, b) over the block; result valid in thread 0
@@ -226,6 +226,34 @@ __device__ __forceinline__ void block_sum2(double& a, double& b, double* red) {
   }
 }
 
+// v (frequency layout) *= a real (W, W) table in natural (ky, kx) order
+template <int W>
+__device__ __forceinline__ void mul_real_table(Win& v, const float* __restrict__ tab) {
+  using G = Geo<W>;
+  const int t = threadIdx.x;
+#pragma unroll
+  for (int j = 0; j < 16; ++j) {
+    const float* m = tab + G::fky(t, 2 * j) * W + G::fkx(t, 2 * j);
+    const float2 mk = make_float2(m[0], m[W / 2]);
+    v.re[j] = pmul(v.re[j], mk);
+    v.im[j] = pmul(v.im[j], mk);
+  }
+}
+
+// v (frequency layout) *= a complex (W, W) table in natural (ky, kx) order, or its conjugate
+template <int W>
+__device__ __forceinline__ void mul_table(Win& v, const float2* __restrict__ tab, bool conj) {
+  using G = Geo<W>;
+  const int t = threadIdx.x;
+#pragma unroll
+  for (int j = 0; j < 16; ++j) {
+    const float2* m = tab + G::fky(t, 2 * j) * W + G::fkx(t, 2 * j);
+    const float2 a = m[0], b = m[W / 2];
+    const float2 py = conj ? make_float2(-a.y, -b.y) : make_float2(a.y, b.y);
+    pcmul(v.re[j], v.im[j], make_float2(a.x, b.x), py, pneg(py));
+  }
+}
+
 // ------------------------------------------------------------------ probe spectrum
 // probe (W, W, Mp) reference layout -> FFT per mode, native frequency layout [Mp]
 template <int W>
@@ -240,11 +268,11 @@ __global__ void __launch_bounds__(Geo<W>::T) probe_fft_kernel(const float2* __re
   load_twiddles<W>(tw1, tw2, g_tw);
   __syncthreads();
   const int t = threadIdx.x, p = blockIdx.x;
-  float2 v[32];
+  Win v;
 #pragma unroll
-  for (int i = 0; i < 32; ++i) v[i] = probe[(size_t)(G::ry(t) * W + G::rx(t, i)) * Mp + p];
+  for (int i = 0; i < 32; ++i) wset(v, i, probe[(size_t)(G::ry(t) * W + G::rx(t, i)) * Mp + p]);
   WinFFT<W>::forward(v, xbuf, tw1, tw2);
-  st_native<W>(probe_f + (size_t)p * W * W, v);
+  st_native(probe_f + (size_t)p * W * W, v);
 }
 
 // ------------------------------------------------------------------ object windows
@@ -274,15 +302,14 @@ __global__ void __launch_bounds__(Geo<W>::T) object_windows_kernel(WindowArgs a)
   const int gi = a.seq[b];
   const int y0 = a.pos[2 * gi], x0 = a.pos[2 * gi + 1];
   const float2* src = a.obj + (size_t)k * a.Ny * a.Nx + (size_t)(y0 + G::ry(t)) * a.Nx + x0;
-  float2 v[32];
+  Win v;
 #pragma unroll
-  for (int i = 0; i < 32; ++i) v[i] = src[G::rx(t, i)];
+  for (int i = 0; i < 32; ++i) wset(v, i, src[G::rx(t, i)]);
   __syncthreads();
   WinFFT<W>::forward(v, xbuf, tw1, tw2);
-#pragma unroll
-  for (int i = 0; i < 32; ++i) v[i] = cscale(v[i], a.mask_sc[G::fky(t, i) * W + G::fkx(t, i)]);
+  mul_real_table<W>(v, a.mask_sc);
   WinFFT<W>::inverse(v, xbuf, tw1, tw2);
-  st_native<W>(a.out + (size_t)win * W * W, v);
+  st_native(a.out + (size_t)win * W * W, v);
 }
 
 // ------------------------------------------------------------------ fused multislice
@@ -312,7 +339,7 @@ struct FusedArgs {
   const int* seq;           // batch's sequence entries
   const float* measured;    // (N, W, W) detector (fftshifted) order
   const float2* tw;
-  float2* stack;            // conj input waves, native real [Bb*Z*Mp*Mo]
+  float2* stack;            // input waves (256 windows: their conjugates), native real [Bb*Z*Mp*Mo]
   float2* gsum;             // object-gradient contributions, native real [Bb*Z*Mo*Mp] (probe mode innermost)
   float2* fprobe;           // FFT of the per-position probe gradient, native freq [Bb*Mp]
   float2* gbuf;             // dL/d(exit wave) between the two halves, native real [Bb*Mp*Mo]
@@ -340,9 +367,9 @@ __device__ __forceinline__ float2 shift_ramp(const FusedArgs& a, int ky, int kx,
 }
 
 // The same ramp for a binary mask, inside the mask: exp(i sx[kx] dx) * exp(i sy[ky] dy). A
-// thread's 32 frequency-layout elements i = q*Bq + r span Q distinct kx (by q) and Bq distinct
-// ky (by r), so Q + Bq sincos evaluations serve all 32 (the caller zeroes the elements outside
-// the mask). f(i, ky, kx, ramp) is called for every element, i a compile-time constant.
+// thread's 32 frequency-layout elements span Q distinct kx and Bq distinct ky, so Q + Bq sincos
+// evaluations serve all 32 (the caller zeroes the elements outside the mask). f(i, ky, kx, ramp)
+// is called for every element, i a compile-time constant.
 template <int W, typename Fn>
 __device__ __forceinline__ void visit_sep_ramp(const FusedArgs& a, int t, float dy, float dx, Fn&& f) {
   using G = Geo<W>;
@@ -352,37 +379,27 @@ __device__ __forceinline__ void visit_sep_ramp(const FusedArgs& a, int t, float 
     sincosf(__fmul_rn(s, d), &sn, &cs);
     return make_float2(cs, sn);
   };
-  if constexpr (Q <= Bq) {   // the Q x factors kept, one y factor at a time
-    float2 ex[Q];
-    static_for<0, Q>([&](auto QQ) {
-      constexpr int q = decltype(QQ)::value;
-      ex[q] = phase(a.sx[G::fkx(t, q * Bq)], dx);
-    });
+  float2 ey[Bq];
+  static_for<0, Bq>([&](auto RR) {
+    constexpr int r = decltype(RR)::value;
+    ey[r] = phase(a.sy[G::fky(t, 2 * r)], dy);
+  });
+  static_for<0, Q>([&](auto QQ) {   // kx number q: half q % 2 of the packs (q / 2) * Bq + r
+    constexpr int q = decltype(QQ)::value, i0 = 2 * (q / 2) * Bq + q % 2;
+    const int kx = G::fkx(t, i0);
+    const float2 ex = phase(a.sx[kx], dx);
     static_for<0, Bq>([&](auto RR) {
-      constexpr int r = decltype(RR)::value;
-      const int ky = G::fky(t, r);
-      const float2 ey = phase(a.sy[ky], dy);
-      static_for<0, Q>([&](auto QQ) {
-        constexpr int q = decltype(QQ)::value;
-        f(std::integral_constant<int, q * Bq + r>{}, ky, G::fkx(t, q * Bq), cmul(ex[q], ey));
-      });
+      constexpr int i = i0 + 2 * decltype(RR)::value;
+      f(std::integral_constant<int, i>{}, G::fky(t, i), kx, cmul(ex, ey[decltype(RR)::value]));
     });
-  } else {                   // the Bq y factors kept, one x factor at a time
-    float2 ey[Bq];
-    static_for<0, Bq>([&](auto RR) {
-      constexpr int r = decltype(RR)::value;
-      ey[r] = phase(a.sy[G::fky(t, r)], dy);
-    });
-    static_for<0, Q>([&](auto QQ) {
-      constexpr int q = decltype(QQ)::value;
-      const int kx = G::fkx(t, q * Bq);
-      const float2 ex = phase(a.sx[kx], dx);
-      static_for<0, Bq>([&](auto RR) {
-        constexpr int r = decltype(RR)::value;
-        f(std::integral_constant<int, q * Bq + r>{}, G::fky(t, r), kx, cmul(ex, ey[r]));
-      });
-    });
-  }
+  });
+}
+
+// Detector (fftshifted) pixel of element i of thread t in the frequency layout.
+template <int W>
+__device__ __forceinline__ int detector_index(int t, int i) {
+  using G = Geo<W>;
+  return ((G::fky(t, i) + W / 2) & (W - 1)) * W + ((G::fkx(t, i) + W / 2) & (W - 1));
 }
 
 // A thread's running sum of float32 terms, compensated: every add is Knuth's TwoSum, so hi + lo
@@ -438,19 +455,19 @@ __device__ __forceinline__ float loss_pixel(int alg, float I, float Mv, Acc& lsu
   return d;
 }
 
-// Shared memory of the fused kernel: the FFT exchange buffer (which also receives each
-// step's main operand by TMA bulk copy), twiddles, reduction scratch, a side buffer for the
-// first NST elements per thread of the adjoint step's object window, and two mbarriers.
+// Shared memory of the fused kernel: the FFT exchange buffer (which also receives the adjoint
+// steps' object windows by TMA bulk copy), twiddles, reduction scratch, a side buffer for the
+// first NST elements per thread of each step's streamed window, and two mbarriers per warp.
 template <int W>
 struct FusedSmem {
   static constexpr int NST = (W == 128) ? 22 : 16;
   static constexpr size_t side_off = Smem<W>::bytes;
   static constexpr size_t pyx_off = side_off + sizeof(float2) * NST * Geo<W>::T;
-  static constexpr size_t bits_off = pyx_off + sizeof(float2) * 2 * W;
+  static constexpr size_t bits_off = pyx_off + sizeof(float2) * 3 * W;   // y factors as packs, x factors
   static constexpr size_t bar_off = bits_off + sizeof(uint32_t) * Geo<W>::T;
   // W = 64: the position's measured pattern (W^2 floats, detector order), copied in at the
   // start, and the probe-shift ramp of the first step (frequency layout), reused by the last
-  static constexpr size_t meas_off = (bar_off + 2 * sizeof(uint64_t) + 15) & ~(size_t)15;
+  static constexpr size_t meas_off = (bar_off + 2 * (Geo<W>::T / 32) * sizeof(uint64_t) + 15) & ~(size_t)15;
   static constexpr size_t ramp_off = meas_off + (W == 64 ? sizeof(float) * W * W : 0);
   static constexpr size_t bytes = ramp_off + (W == 64 ? sizeof(float2) * W * W : 0);
 };
@@ -465,18 +482,20 @@ struct FusedSmem {
 // inverse FFT", so the forward and inverse transforms are each inlined once and the window
 // never leaves the registers:
 //   step 0          incoming probe (shift ramp in frequency, inverse FFT)
-//   steps 1..Z      slice z = s-1: store conj(psi_z), psi *= O_z, FFT, *= P (or the far
+//   steps 1..Z      slice z = s-1: store psi_z, psi *= O_z, FFT, *= P (or the far
 //                   field, loss and dL/dPsi after the last slice), IFFT
 //   steps Z+1..2Z   slice z = 2Z-s: object-gradient contribution, g *= conj(O_z), FFT,
 //                   *= conj(P), IFFT (z = 0: probe-gradient spectrum and position gradient)
-// Operands: the side buffer (each thread's first NST elements, a prefix of the native layout)
-// takes every step's streamed window by TMA one step ahead -- O_z in the forward, conj(psi_z)
-// from the stack in the adjoint -- and the rest of that window is loaded at the step. The step
-// writes its outgoing window (conj(psi_z) in the forward, this mode's gradient contribution in
-// the adjoint) into the side buffer in place of what it read, and a TMA bulk store takes it out
-// behind the forward transform. The adjoint's O_z lands in the exchange buffer while the
+// Operands: every warp moves its own share of each window (8 KB in the native layout) through
+// its own parts of the side and exchange buffers, with its own mbarriers, so no operand waits on
+// a block barrier. The side buffer (each thread's first NST elements) takes every step's
+// streamed window by TMA one step ahead -- O_z in the forward, conj(psi_z) from the stack in the
+// adjoint -- and the rest of that window is loaded at the step. The step writes its outgoing
+// window (psi_z in the forward, this mode's gradient contribution in the adjoint) into the
+// side buffer in place of what it read, and a TMA bulk store takes it out behind the forward
+// transform. The adjoint's O_z lands in the warp's part of the exchange buffer while the
 // inverse transform finishes its last register-only round; the adjoint's first step finds
-// conj(psi_{Z-1}) still in the side buffer.
+// psi_{Z-1} still in the side buffer.
 // PH = 0: the whole pass (phase 0) with every phase branch compiled out; PH = 1: a.phase at
 // run time (the split halves and the multislice_core phases).
 template <int W, int PH>
@@ -497,12 +516,14 @@ __global__ void __launch_bounds__(Geo<W>::T, Geo<W>::MINB) fused_multislice_kern
   double* red;
   carve<W>(smem, xbuf, tw1, tw2, red);
   float2* side = reinterpret_cast<float2*>(smem + S::side_off);
-  float2* spy = reinterpret_cast<float2*>(smem + S::pyx_off);   // [W] y factor, then [W] x factor
-  const float2* spx = spy + W;
+  float4* spy = reinterpret_cast<float4*>(smem + S::pyx_off);   // [W] y factor (re, re, im, im)
+  float2* spx = reinterpret_cast<float2*>(spy + W);             // [W] x factor
   uint32_t* sbits = reinterpret_cast<uint32_t*>(smem + S::bits_off);
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + S::bar_off);   // [0]: xbuf, [1]: side
-  float* fs0 = reinterpret_cast<float*>(xbuf);   // WW floats: this block's |Psi|^2
-  float* fs1 = fs0 + WW;                          // WW floats: mode-summed I, then dL/dI
+  constexpr int NW = T / 32;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + S::bar_off);   // per warp: xbuf parts, then side parts
+  // per pack, in the order of the threads' packs [16][T]
+  float2* fs0 = xbuf;              // this block's |Psi|^2
+  float2* fs1 = fs0 + WW / 2;      // mode-summed I, then dL/dI
   cg::cluster_group cluster = cg::this_cluster();
   const int t = threadIdx.x;
   const int nmodes = a.Mp * a.Mo;
@@ -512,15 +533,24 @@ __global__ void __launch_bounds__(Geo<W>::T, Geo<W>::MINB) fused_multislice_kern
   const int gi = a.seq[b];
   const float dy = a.corr[2 * gi], dx = a.corr[2 * gi + 1];
   const int Z = a.Z;
-  const bool adj_stack = a.step_obj && !a.simulate;   // the adjoint reads conj(psi_z)
+  const bool adj_stack = a.step_obj && !a.simulate;   // the adjoint reads psi_z
   const int phase = PH == 0 ? 0 : a.phase;
-  if (t == 0) {
-    mbar_init(&bars[0], 1);
-    mbar_init(&bars[1], 1);
+  const int warp = t >> 5, lane = t & 31;
+  uint64_t *bar_x = bars + warp, *bar_side = bars + NW + warp;
+  float4* wx = reinterpret_cast<float4*>(xbuf + warp * F::WPART);         // this warp's share of xbuf
+  float4* wside = reinterpret_cast<float4*>(side) + warp * (NST / 2 * 32);   // and of the side buffer
+  const int wo = nword(0, t);   // this thread's first 16-byte word of a native window
+  if (lane == 0) {
+    mbar_init(bar_x, 1);
+    mbar_init(bar_side, 1);
     fence_async_shared();
   }
   load_twiddles<W>(tw1, tw2, a.tw);
-  for (int i = t; i < 2 * W; i += T) spy[i] = a.pyx[i];
+  for (int i = t; i < W; i += T) {
+    const float2 y = a.pyx[i];
+    spy[i] = make_float4(y.x, y.x, y.y, y.y);
+    spx[i] = a.pyx[W + i];
+  }
   // bit i: element i (frequency layout) of this thread lies inside the band limit
   {
     uint32_t mbits = 0;
@@ -550,37 +580,64 @@ __global__ void __launch_bounds__(Geo<W>::T, Geo<W>::MINB) fused_multislice_kern
   // O_z of step s >= 1: the adjoint steps read it from the exchange buffer, the forward steps
   // through the side buffer
   auto xsrc = [&](int s) -> const float2* { return obl_ptr(s <= Z ? s - 1 : 2 * Z - s); };
+  // (the warp has finished with the destination and passed a __syncwarp)
   auto issue_x = [&](int s) {
-    if (t == 0) {
+    if (lane == 0) {
       fence_async_shared();
-      bulk_load(xbuf, xsrc(s), (uint32_t)(WW * sizeof(float2)), &bars[0]);
+      bulk_load(wx, xsrc(s) + warp * F::WPART, (uint32_t)(F::WPART * sizeof(float2)), bar_x);
     }
   };
-  constexpr uint32_t kSideBytes = (uint32_t)(NST * T * sizeof(float2));
-  // the side buffer takes the first NST elements per thread (a prefix of the native layout) of
-  // a window: O_z in the forward, conj(psi_z) from the stack in the adjoint
+  constexpr uint32_t kSideBytes = (uint32_t)(NST * 32 * sizeof(float2));
+  // the side buffer takes the first NST elements per thread of a window: O_z in the forward,
+  // psi_z from the stack in the adjoint
   auto issue_side = [&](const float2* src) {
-    if (t == 0) {
+    if (lane == 0) {
       fence_async_shared();
-      bulk_load(side, src, kSideBytes, &bars[1]);
+      bulk_load(wside, src + warp * F::WPART, kSideBytes, bar_side);
     }
   };
-  // the window that the staged side buffer goes to: code z < Z is the stack window of slice z
-  // (forward), code Z + z this mode's gradient contribution of slice z (adjoint)
   auto contrib_ptr = [&](int z) { return a.gsum + ((((size_t)b * Z + z) * a.Mo + m) * a.Mp + p) * WW; };
-  auto store_ptr = [&](int code) { return code < Z ? stack_ptr(code) : contrib_ptr(code - Z); };
+  // the staged part of the side buffer leaves for the window `dst` by a bulk store
+  auto store_side = [&](float2* dst) {
+    fence_async_shared();
+    __syncwarp();
+    if (lane == 0) bulk_store(dst + warp * F::WPART, wside, kSideBytes);
+  };
 
-  float2 v[32];
+  // v *= P or conj(P) inside the band limit, zero outside, P = P_y(ky) P_x(kx)
+  auto propagate_sep = [&](Win& v, bool conj) {
+    const uint32_t mbits = sbits[t];
+    constexpr int NQ = G::Q / 2;
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) {
+      const int kx = G::fkx(t, 2 * q * G::Bq);
+      const float2 xa = spx[kx], xb = spx[kx + W / 2];
+      const float2 xr = make_float2(xa.x, xb.x), xi = make_float2(xa.y, xb.y), nxi = pneg(xi);
+#pragma unroll
+      for (int r = 0; r < G::Bq; ++r) {
+        const int j = q * G::Bq + r;
+        const float4 y = spy[G::fky(t, 2 * j)];
+        const float2 yr = make_float2(y.x, y.y), yi = make_float2(y.z, y.w);
+        const float2 pr = pfma(yi, nxi, pmul(yr, xr));
+        const float2 pi = pfma(yi, xr, pmul(yr, xi)), ni = pneg(pi);
+        pcmul(v.re[j], v.im[j], pr, conj ? ni : pi, conj ? pi : ni);
+        const bool in0 = (mbits >> (2 * j)) & 1u, in1 = (mbits >> (2 * j + 1)) & 1u;
+        v.re[j] = make_float2(in0 ? v.re[j].x : 0.f, in1 ? v.re[j].y : 0.f);
+        v.im[j] = make_float2(in0 ? v.im[j].x : 0.f, in1 ? v.im[j].y : 0.f);
+      }
+    }
+  };
+
+  Win v;
   int side_next = -1;        // the slice whose window prefix the side buffer takes next
   bool side_held = false;    // the side buffer holds the next step's operand, waited for
-  int store_code = -1;       // the side buffer is staged for a bulk store to store_ptr(store_code)
   float2* gb = a.gbuf + (((size_t)b * a.Mp + p) * a.Mo + m) * WW;
   const bool adjoint_only = (phase == 2 || phase == 4);
   const int s_begin = adjoint_only ? Z + 1 : 0;
   const int s_end = (a.simulate || phase == 1 || phase == 3) ? Z + 1 : 2 * Z + 1;
   if (adjoint_only) {
     // adjoint half: resume from dL/d(exit wave) kept by the forward half
-    ld_native<W>(gb, v);
+    ld_native(gb, v);
     issue_x(Z + 1);
     if (adj_stack) issue_side(stack_ptr(Z - 1));
   } else {
@@ -593,10 +650,10 @@ __global__ void __launch_bounds__(Geo<W>::T, Geo<W>::MINB) fused_multislice_kern
     // ------------------------------------------------ real-space op
     if (s == 0) {
       if (PH != 0 && a.probe_b) {
-        ld_native<W>(a.probe_b + ((size_t)b * a.Mp + p) * WW, v);
+        ld_native(a.probe_b + ((size_t)b * a.Mp + p) * WW, v);
       } else if (!a.probe_shift) {
 #pragma unroll
-        for (int i = 0; i < 32; ++i) v[i] = a.probe[(size_t)(G::ry(t) * W + G::rx(t, i)) * a.Mp + p];
+        for (int i = 0; i < 32; ++i) wset(v, i, a.probe[(size_t)(G::ry(t) * W + G::rx(t, i)) * a.Mp + p]);
       }
     } else if (fwd) {
       // O_z: elements NST.. straight from global memory (issued first), the rest from the side
@@ -605,75 +662,70 @@ __global__ void __launch_bounds__(Geo<W>::T, Geo<W>::MINB) fused_multislice_kern
       {
         const float4* og = reinterpret_cast<const float4*>(obl_ptr(z));
 #pragma unroll
-        for (int j = NST / 2; j < 16; ++j) otail[j - NST / 2] = og[j * T + t];
+        for (int j = NST / 2; j < 16; ++j) otail[j - NST / 2] = og[wo + j * 32];
       }
-      float4* sd = reinterpret_cast<float4*>(side);
       float4* st = adj_stack ? reinterpret_cast<float4*>(stack_ptr(z)) : nullptr;
-      mbar_wait(&bars[1], ph_side, a.err);
+      mbar_wait(bar_side, ph_side, a.err);
 #pragma unroll
       for (int j = 0; j < 16; ++j) {
-        const float4 q = (j < NST / 2) ? sd[j * T + t] : otail[j - NST / 2];
+        const float4 q = (j < NST / 2) ? wside[j * 32 + lane] : otail[j - NST / 2];
         if (adj_stack) {
-          // conj(psi_z) to the stack: elements < NST in place of O_z in the side buffer, whence
-          // a bulk copy takes them out behind the transform; the rest straight from the registers
-          const float4 c = make_float4(v[2 * j].x, -v[2 * j].y, v[2 * j + 1].x, -v[2 * j + 1].y);
-          if (j < NST / 2) sd[j * T + t] = c;
-          else st[j * T + t] = c;
+          // psi_z to the stack: elements < NST in place of O_z in the side buffer, whence a bulk
+          // copy takes them out behind the transform; the rest straight from the registers
+          const float4 c = pack4(v.re[j], v.im[j]);
+          if (j < NST / 2) wside[j * 32 + lane] = c;
+          else st[wo + j * 32] = c;
         }
-        v[2 * j] = cmul(v[2 * j], make_float2(q.x, q.y));
-        v[2 * j + 1] = cmul(v[2 * j + 1], make_float2(q.z, q.w));
+        const float2 oi = make_float2(q.z, q.w);
+        pcmul(v.re[j], v.im[j], make_float2(q.x, q.y), oi, pneg(oi));
       }
-      if (adj_stack) {
-        fence_async_shared();
-        // the adjoint's first step (the same slice) reads conj(psi_z) from the side buffer itself
-        if (!(z == Z - 1 && phase == 0)) store_code = z;
-      }
+      // the adjoint's first step (the same slice) reads psi_z from the side buffer itself
+      if (adj_stack && !(z == Z - 1 && phase == 0)) store_side(stack_ptr(z));
       if (z + 1 < Z) side_next = z + 1;
       else side_held = true;
       if (phase == 3 && z == Z - 1) {
-        st_native<W>(a.exit_out + (((size_t)b * a.Mp + p) * a.Mo + m) * WW, v);   // the exit wave
+        st_native(a.exit_out + (((size_t)b * a.Mp + p) * a.Mo + m) * WW, v);   // the exit wave
         break;
       }
     } else {
       if (adj_stack) {
-        // conj(psi_z): elements NST.. straight from global memory (this thread stored them in
+        // psi_z: elements NST.. straight from global memory (this thread stored them in
         // the forward), the rest in the side buffer
         float4 stail[(32 - NST) / 2];
         {
           const float4* sg = reinterpret_cast<const float4*>(stack_ptr(z));
 #pragma unroll
-          for (int j = NST / 2; j < 16; ++j) stail[j - NST / 2] = sg[j * T + t];
+          for (int j = NST / 2; j < 16; ++j) stail[j - NST / 2] = sg[wo + j * 32];
         }
         if (side_held) side_held = false;
-        else mbar_wait(&bars[1], ph_side, a.err);
+        else mbar_wait(bar_side, ph_side, a.err);
         // contribution conj(psi_z) * g of this probe mode, to its own window of the gradient
         // buffer ([position][slice][object mode][probe mode]); grad_windows_kernel adds the
         // probe modes in ascending order before the band limit (multislice_core.py:184-191), so
         // the adjoint needs no cluster barrier and no remote reads. Elements < NST replace
-        // conj(psi_z) in the side buffer, whence a bulk copy takes them out behind the transform.
+        // psi_z in the side buffer, whence a bulk copy takes them out behind the transform.
         float4* g4 = reinterpret_cast<float4*>(contrib_ptr(z));
-        float4* sd = reinterpret_cast<float4*>(side);
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
-          const float4 q = (j < NST / 2) ? sd[j * T + t] : stail[j - NST / 2];
-          const float2 g0 = cmul(make_float2(q.x, q.y), v[2 * j]);
-          const float2 g1 = cmul(make_float2(q.z, q.w), v[2 * j + 1]);
-          if (j < NST / 2) sd[j * T + t] = make_float4(g0.x, g0.y, g1.x, g1.y);
-          else g4[j * T + t] = make_float4(g0.x, g0.y, g1.x, g1.y);
+          const float4 q = (j < NST / 2) ? wside[j * 32 + lane] : stail[j - NST / 2];
+          // conj(psi) * g
+          const float2 pr = make_float2(q.x, q.y), pi = make_float2(q.z, q.w);
+          const float2 gr = pfma(v.im[j], pi, pmul(v.re[j], pr));
+          const float2 gi = pfma(v.im[j], pr, pneg(pmul(v.re[j], pi)));
+          if (j < NST / 2) wside[j * 32 + lane] = pack4(gr, gi);
+          else g4[wo + j * 32] = pack4(gr, gi);
         }
-        fence_async_shared();
-        store_code = Z + z;
+        store_side(contrib_ptr(z));
         if (z > 0) side_next = z - 1;
       }
       // g *= conj(O_z), O_z in the exchange buffer
-      mbar_wait(&bars[0], ph_x, a.err);
+      mbar_wait(bar_x, ph_x, a.err);
       {
-        const float4* ob = reinterpret_cast<const float4*>(xbuf);
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
-          const float4 q = ob[j * T + t];
-          v[2 * j] = cmulc(v[2 * j], make_float2(q.x, q.y));
-          v[2 * j + 1] = cmulc(v[2 * j + 1], make_float2(q.z, q.w));
+          const float4 q = wx[j * 32 + lane];
+          const float2 oi = make_float2(q.z, q.w);
+          pcmul(v.re[j], v.im[j], make_float2(q.x, q.y), pneg(oi), oi);
         }
       }
       if (z == 0) {
@@ -682,7 +734,7 @@ __global__ void __launch_bounds__(Geo<W>::T, Geo<W>::MINB) fused_multislice_kern
           // probe gradient: sum over object modes (multislice_core.py:193-197)
           __syncthreads();
 #pragma unroll
-          for (int i = 0; i < 32; ++i) xbuf[i * T + t] = v[i];
+          for (int i = 0; i < 32; ++i) xbuf[i * T + t] = wget(v, i);
           cluster.sync();
           if (m == 0) {
 #pragma unroll
@@ -690,14 +742,14 @@ __global__ void __launch_bounds__(Geo<W>::T, Geo<W>::MINB) fused_multislice_kern
               float2 acc = make_float2(0.f, 0.f);
               for (int mm = 0; mm < a.Mo; ++mm)
                 acc = cadd(acc, cluster.map_shared_rank(xbuf, p + mm * a.Mp)[i * T + t]);
-              v[i] = acc;
+              wset(v, i, acc);
             }
           }
           cluster.sync();
           if (m != 0) break;
         }
         if (phase == 4) {   // interm_probe_grad of multislice_core.py:193-197, real space
-          if (a.step_probe) st_native<W>(a.fprobe + ((size_t)b * a.Mp + p) * WW, v);
+          if (a.step_probe) st_native(a.fprobe + ((size_t)b * a.Mp + p) * WW, v);
           break;
         }
       }
@@ -705,22 +757,11 @@ __global__ void __launch_bounds__(Geo<W>::T, Geo<W>::MINB) fused_multislice_kern
 
     // ------------------------------------------------ forward FFT
     if (s > 0) {
-      F::forward_round1(v, tw1);
-      const bool staged = store_code >= 0;
-      auto side_src = [&](int zz) { return fwd ? obl_ptr(zz) : stack_ptr(zz); };
-      F::forward_rest(v, xbuf, tw1, tw2, [&] {
-        // every thread has finished with the side buffer: copy its staged part out, or refill it
-        if (staged) {
-          if (t == 0) bulk_store(store_ptr(store_code), side, kSideBytes);
-          store_code = -1;
-        } else if (side_next >= 0) {
-          issue_side(side_src(side_next));
-          side_next = -1;
-        }
-      });
-      if (side_next >= 0) {   // refill the side buffer once the bulk store has read it
-        if (t == 0) bulk_wait_read();
-        issue_side(side_src(side_next));
+      __syncwarp();   // the warp has read its operands from the exchange and side buffers
+      F::forward(v, xbuf, tw1, tw2);
+      if (side_next >= 0) {   // refill the side buffer once its bulk store has read it
+        if (lane == 0) bulk_wait_read();
+        issue_side(fwd ? obl_ptr(side_next) : stack_ptr(side_next));
         side_next = -1;
       }
     }
@@ -734,29 +775,23 @@ __global__ void __launch_bounds__(Geo<W>::T, Geo<W>::MINB) fused_multislice_kern
         const uint32_t mbits = sbits[t];
         visit_sep_ramp<W>(a, t, dy, dx, [&](auto I, int, int, float2 ramp) {
           constexpr int i = decltype(I)::value;
-          v[i] = ((mbits >> i) & 1u) ? cscale(cmul(pf[nidx<W>(i, t)], ramp), inv) : make_float2(0.f, 0.f);
+          wset(v, i, ((mbits >> i) & 1u) ? cscale(cmul(native_at(pf, i, t), ramp), inv) : make_float2(0.f, 0.f));
           sramp[i * T + t] = ramp;   // the same ramp serves the probe-gradient step (phase 0)
         });
       } else {
 #pragma unroll
         for (int i = 0; i < 32; ++i) {
           const int ky = G::fky(t, i), kx = G::fkx(t, i);
-          v[i] = cscale(cmul(pf[nidx<W>(i, t)], shift_ramp<W>(a, ky, kx, a.mask[ky * W + kx], dy, dx)), inv);
+          wset(v, i, cscale(cmul(native_at(pf, i, t), shift_ramp<W>(a, ky, kx, a.mask[ky * W + kx], dy, dx)), inv));
         }
       }
     } else if (fwd && z < Z - 1) {
       if (a.use_sep && !(z == 0 && a.use_edge)) {
-        const uint32_t mbits = sbits[t];
-#pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          const float2 P = cmul(spy[G::fky(t, i)], spx[G::fkx(t, i)]);
-          v[i] = ((mbits >> i) & 1u) ? cmul(v[i], P) : make_float2(0.f, 0.f);
-        }
+        propagate_sep(v, false);
       } else {
         const float2* pr = a.prop_steps ? a.prop_steps + (size_t)z * WW
                                         : ((z == 0 && a.use_edge) ? a.prop_edge : a.prop);
-#pragma unroll
-        for (int i = 0; i < 32; ++i) v[i] = cmul(v[i], pr[G::fky(t, i) * W + G::fkx(t, i)]);
+        mul_table<W>(v, pr, false);
       }
     } else if (fwd) {
       // far field: Psi = FFT(exit) * mask, I = mean over modes |Psi|^2 (objective.py:501-512)
@@ -766,33 +801,32 @@ __global__ void __launch_bounds__(Geo<W>::T, Geo<W>::MINB) fused_multislice_kern
       if (kLean && a.mask_bin) {
         const uint32_t mbits = sbits[t];
 #pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          if (!((mbits >> i) & 1u)) v[i] = make_float2(0.f, 0.f);
-          fs0[i * T + t] = cabs2(v[i]);
+        for (int j = 0; j < 16; ++j) {
+          const bool in0 = (mbits >> (2 * j)) & 1u, in1 = (mbits >> (2 * j + 1)) & 1u;
+          v.re[j] = make_float2(in0 ? v.re[j].x : 0.f, in1 ? v.re[j].y : 0.f);
+          v.im[j] = make_float2(in0 ? v.im[j].x : 0.f, in1 ? v.im[j].y : 0.f);
         }
       } else {
-#pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          v[i] = cscale(v[i], a.mask[G::fky(t, i) * W + G::fkx(t, i)]);
-          fs0[i * T + t] = cabs2(v[i]);
-        }
+        mul_real_table<W>(v, a.mask);
       }
+#pragma unroll
+      for (int j = 0; j < 16; ++j) fs0[j * T + t] = pfma(v.im[j], v.im[j], pmul(v.re[j], v.re[j]));
       cluster.sync();
 #pragma unroll 1
-      for (int i0 = 0; i0 < 32; i0 += 8) {
-        float acc[8];
+      for (int j0 = 0; j0 < 16; j0 += 4) {
+        float2 acc[4];
 #pragma unroll
-        for (int k = 0; k < 8; ++k) acc[k] = 0.0f;
+        for (int k = 0; k < 4; ++k) acc[k] = make_float2(0.f, 0.f);
 #pragma unroll
         for (int r = 0; r < 8; ++r) {      // ranks in ascending order: a fixed summation order
           if (r < nmodes) {
-            const float* rb = cluster.map_shared_rank(fs0, r);
+            const float2* rb = cluster.map_shared_rank(fs0, r);
 #pragma unroll
-            for (int k = 0; k < 8; ++k) acc[k] += rb[(i0 + k) * T + t];
+            for (int k = 0; k < 4; ++k) acc[k] = padd(acc[k], rb[(j0 + k) * T + t]);
           }
         }
 #pragma unroll
-        for (int k = 0; k < 8; ++k) fs1[(i0 + k) * T + t] = acc[k];
+        for (int k = 0; k < 4; ++k) fs1[(j0 + k) * T + t] = acc[k];
       }
       cluster.sync();   // every block is done reading this block's intensities
       const float inv_modes = 1.0f / (float)nmodes;
@@ -803,9 +837,7 @@ __global__ void __launch_bounds__(Geo<W>::T, Geo<W>::MINB) fused_multislice_kern
       auto load8 = [&](int i0, float (&dst)[8]) {
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
-          const int i = i0 + k;
-          const int ky = G::fky(t, i), kx = G::fkx(t, i);
-          const int didx = ((ky + W / 2) & (W - 1)) * W + ((kx + W / 2) & (W - 1));
+          const int didx = detector_index<W>(t, i0 + k);
           dst[k] = a.simulate ? 0.0f : (kLean ? smeas[didx] : meas[didx]);
         }
       };
@@ -819,19 +851,26 @@ __global__ void __launch_bounds__(Geo<W>::T, Geo<W>::MINB) fused_multislice_kern
           load8(i0, mv);
         }
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          const int i = i0 + k;
-          const float acc = fs1[i * T + t];
-          const float I = (nmodes == 1) ? acc : acc * inv_modes;
+        for (int k = 0; k < 8; k += 2) {
+          const float2 acc = fs1[((i0 + k) >> 1) * T + t];
+          const float I0 = (nmodes == 1) ? acc.x : acc.x * inv_modes;
+          const float I1 = (nmodes == 1) ? acc.y : acc.y * inv_modes;
           if (a.simulate) {
-            const int ky = G::fky(t, i), kx = G::fkx(t, i);
-            const int didx = ((ky + W / 2) & (W - 1)) * W + ((kx + W / 2) & (W - 1));
-            if (crank == 0) a.sim_out[(size_t)b * WW + didx] = I;
+            if (crank == 0) {
+              float* so = a.sim_out + (size_t)b * WW;
+              so[detector_index<W>(t, i0 + k)] = I0;
+              so[detector_index<W>(t, i0 + k + 1)] = I1;
+            }
             continue;
           }
-          float d = loss_pixel(a.algorithm, I, mv[k], lsum_c, ssum_c);
-          if (nmodes > 1) d = d / (float)nmodes;           // objective.py:586-587
-          fs1[i * T + t] = d;
+          float2 d;
+          d.x = loss_pixel(a.algorithm, I0, mv[k], lsum_c, ssum_c);
+          d.y = loss_pixel(a.algorithm, I1, mv[k + 1], lsum_c, ssum_c);
+          if (nmodes > 1) {                                // objective.py:586-587
+            d.x = d.x / (float)nmodes;
+            d.y = d.y / (float)nmodes;
+          }
+          fs1[((i0 + k) >> 1) * T + t] = d;
         }
         if constexpr (kLean) {
 #pragma unroll
@@ -847,20 +886,19 @@ __global__ void __launch_bounds__(Geo<W>::T, Geo<W>::MINB) fused_multislice_kern
       }
       // dL/dPsi = dLdI * Psi * (w * W^2); the W^2 cancels the 1/W^2 of ifft2 (objective.py:595-597)
 #pragma unroll
-      for (int i = 0; i < 32; ++i) v[i] = cscale(cscale(v[i], fs1[i * T + t]), a.loss_weight);
+      for (int j = 0; j < 16; ++j) {
+        const float2 d = fs1[j * T + t], lw = pdup(a.loss_weight);
+        v.re[j] = pmul(pmul(v.re[j], d), lw);
+        v.im[j] = pmul(pmul(v.im[j], d), lw);
+      }
+      __syncthreads();   // the inverse transform's stores replace other threads' dL/dI
     } else if (z > 0) {
       if (a.use_sep && !(z == 1 && a.use_edge)) {
-        const uint32_t mbits = sbits[t];
-#pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          const float2 P = cmul(spy[G::fky(t, i)], spx[G::fkx(t, i)]);
-          v[i] = ((mbits >> i) & 1u) ? cmulc(v[i], P) : make_float2(0.f, 0.f);
-        }
+        propagate_sep(v, true);
       } else {
         const float2* pr = a.prop_steps ? a.prop_steps + (size_t)(z - 1) * WW
                                         : ((z == 1 && a.use_edge) ? a.prop_edge : a.prop);
-#pragma unroll
-        for (int i = 0; i < 32; ++i) v[i] = cmulc(v[i], pr[G::fky(t, i) * W + G::fkx(t, i)]);
+        mul_table<W>(v, pr, true);
       }
     } else {
       // probe-gradient spectrum with the shift adjoint, position gradient (objective.py:641-656)
@@ -873,9 +911,10 @@ __global__ void __launch_bounds__(Geo<W>::T, Geo<W>::MINB) fused_multislice_kern
         for (int i = 0; i < 32; ++i) {
           const int ky = G::fky(t, i), kx = G::fkx(t, i);
           const float mk = ((mbits >> i) & 1u) ? 1.0f : 0.0f;
-          v[i] = cmulc(v[i], cscale(sramp[i * T + t], mk));
+          const float2 g = cmulc(wget(v, i), cscale(sramp[i * T + t], mk));
+          wset(v, i, g);
           if (a.step_pos) {   // as below
-            const float im = cmulc(v[i], pf[nidx<W>(i, t)]).y;
+            const float im = cmulc(g, native_at(pf, i, t)).y;
             gy_c += -(a.sy[ky] * mk) * im;
             gx_c += -(a.sx[kx] * mk) * im;
           }
@@ -885,16 +924,17 @@ __global__ void __launch_bounds__(Geo<W>::T, Geo<W>::MINB) fused_multislice_kern
         for (int i = 0; i < 32; ++i) {
           const int ky = G::fky(t, i), kx = G::fkx(t, i);
           const float mk = a.mask[ky * W + kx];
-          v[i] = cmulc(v[i], shift_ramp<W>(a, ky, kx, mk, dy, dx));
+          const float2 g = cmulc(wget(v, i), shift_ramp<W>(a, ky, kx, mk, dy, dx));
+          wset(v, i, g);
           if (a.step_pos) {
             // Re(smyx * conj(Pf) * F) with smyx = i*s*mask  ->  -(s*mask) * Im(conj(Pf) * F)
-            const float im = cmulc(v[i], pf[nidx<W>(i, t)]).y;
+            const float im = cmulc(g, native_at(pf, i, t)).y;
             gy_c += -(a.sy[ky] * mk) * im;
             gx_c += -(a.sx[kx] * mk) * im;
           }
         }
       }
-      if (a.step_probe) st_native<W>(a.fprobe + ((size_t)b * a.Mp + p) * WW, v);
+      if (a.step_probe) st_native(a.fprobe + ((size_t)b * a.Mp + p) * WW, v);
       if (a.step_pos) {
         double gy = gy_c.value(), gx = gx_c.value();
         block_sum2(gy, gx, red);
@@ -911,9 +951,9 @@ __global__ void __launch_bounds__(Geo<W>::T, Geo<W>::MINB) fused_multislice_kern
     F::inverse_head(v, xbuf, tw1, tw2);
     if (s + 1 < s_end) {
       if (s + 1 > Z) {     // the adjoint steps read O_z from the exchange buffer
-        __syncthreads();   // every thread has finished reading it
+        __syncwarp();      // the warp has finished reading its part
         // the adjoint's side-buffer copies read the stack's bulk-stored parts back
-        if (s == Z && t == 0) bulk_wait_all();
+        if (s == Z && lane == 0) bulk_wait_all();
         issue_x(s + 1);
       }
       // every block asks for its operands at about the same time: bring what the next steps
@@ -921,51 +961,53 @@ __global__ void __launch_bounds__(Geo<W>::T, Geo<W>::MINB) fused_multislice_kern
       // O_z two steps ahead (copied into the exchange buffer just in time) and the parts of the
       // side-buffer windows that are read by plain loads (their prefixes arrive by TMA a whole
       // step ahead)
-      if (t == 0) {
-        constexpr uint32_t kTailBytes = (uint32_t)((WW - (size_t)NST * T) * sizeof(float2));
+      if (lane == 0) {
+        constexpr uint32_t kTailBytes = (uint32_t)((32 - NST) * 32 * sizeof(float2));
         if (s + 2 < s_end) {
+          const float2* src = xsrc(s + 2) + warp * F::WPART;
           if (s + 2 <= Z)   // forward: the side copy (a step ahead) takes the prefix; the tail is loaded
-            prefetch_l2(xsrc(s + 2) + (size_t)NST * T, kTailBytes);
+            prefetch_l2(src + NST * 32, kTailBytes);
           else              // adjoint: O_z goes to the exchange buffer just in time
-            prefetch_l2(xsrc(s + 2), (uint32_t)(WW * sizeof(float2)));
+            prefetch_l2(src, (uint32_t)(F::WPART * sizeof(float2)));
         }
         const int zs = 2 * Z - s - 2;
-        if (adj_stack && s >= Z && zs >= 0) prefetch_l2(stack_ptr(zs) + (size_t)NST * T, kTailBytes);
+        if (adj_stack && s >= Z && zs >= 0) prefetch_l2(stack_ptr(zs) + warp * F::WPART + NST * 32, kTailBytes);
       }
     }
-    F::inverse_tail(v, tw1);
+    F::inverse_tail(v);
   }
-  if (store_code >= 0) {   // staged by a step that left the loop before its forward transform
-    __syncthreads();
-    if (t == 0) bulk_store(store_ptr(store_code), side, kSideBytes);
-  }
-  if (t == 0) bulk_wait_all();   // the bulk stores are complete before the block exits
-  if (phase == 1) st_native<W>(gb, v);   // forward half: keep dL/d(exit wave)
+  if (lane == 0) bulk_wait_all();   // the bulk stores are complete before the block exits
+  if (phase == 1) st_native(gb, v);   // forward half: keep dL/d(exit wave)
 }
 
 // ------------------------------------------------------------------ reference-layout windows
 // (B, W, W, K) arrays with the mode axes innermost (the reference's layout) <-> the native
-// window layout [B*K] used by the kernels; one block per window.
+// window layout [B*K] used by the kernels, conjugated if conj (the reference keeps conjugated
+// waves); one block per window.
 template <int W>
 __global__ void __launch_bounds__(Geo<W>::T) ref_to_native_kernel(const float2* __restrict__ src,
-                                                                  float2* __restrict__ dst, int K) {
+                                                                  float2* __restrict__ dst, int K, int conj) {
   using G = Geo<W>;
   const int t = threadIdx.x, win = blockIdx.x, b = win / K, k = win % K;
-  float2 v[32];
+  Win v;
 #pragma unroll
-  for (int i = 0; i < 32; ++i) v[i] = src[(((size_t)b * W + G::ry(t)) * W + G::rx(t, i)) * K + k];
-  st_native<W>(dst + (size_t)win * W * W, v);
+  for (int i = 0; i < 32; ++i) {
+    const float2 x = src[(((size_t)b * W + G::ry(t)) * W + G::rx(t, i)) * K + k];
+    wset(v, i, conj ? cconj(x) : x);
+  }
+  st_native(dst + (size_t)win * W * W, v);
 }
 
 template <int W>
 __global__ void __launch_bounds__(Geo<W>::T) native_to_ref_kernel(const float2* __restrict__ src,
-                                                                  float2* __restrict__ dst, int K) {
+                                                                  float2* __restrict__ dst, int K, int conj) {
   using G = Geo<W>;
   const int t = threadIdx.x, win = blockIdx.x, b = win / K, k = win % K;
-  float2 v[32];
-  ld_native<W>(src + (size_t)win * W * W, v);
+  Win v;
+  ld_native(src + (size_t)win * W * W, v);
 #pragma unroll
-  for (int i = 0; i < 32; ++i) dst[(((size_t)b * W + G::ry(t)) * W + G::rx(t, i)) * K + k] = v[i];
+  for (int i = 0; i < 32; ++i)
+    dst[(((size_t)b * W + G::ry(t)) * W + G::rx(t, i)) * K + k] = conj ? cconj(wget(v, i)) : wget(v, i);
 }
 
 // (B, W*W, K) -> (B, K, W*W): per-position windows to per-plane natural windows
@@ -1024,25 +1066,24 @@ __global__ void __launch_bounds__(Geo<W>::T) grad_windows_kernel(float2* buf, co
   load_twiddles<W>(tw1, tw2, g_tw);
   const int t = threadIdx.x;
   float2* win = buf + (size_t)blockIdx.x * nsum * W * W;
-  float2 v[32];
-  ld_native<W>(win, v);
+  Win v;
+  ld_native(win, v);
   for (int p = 1; p < nsum; ++p) {
-    const float4* src = reinterpret_cast<const float4*>(win + (size_t)p * W * W);
+    const float4* src = reinterpret_cast<const float4*>(win + (size_t)p * W * W) + nword(0, t);
 #pragma unroll
     for (int j = 0; j < 16; ++j) {
-      const float4 q = src[j * G::T + t];
-      v[2 * j] = cadd(v[2 * j], make_float2(q.x, q.y));
-      v[2 * j + 1] = cadd(v[2 * j + 1], make_float2(q.z, q.w));
+      const float4 q = src[j * 32];
+      v.re[j] = padd(v.re[j], make_float2(q.x, q.y));
+      v.im[j] = padd(v.im[j], make_float2(q.z, q.w));
     }
   }
   __syncthreads();
   WinFFT<W>::forward(v, xbuf, tw1, tw2);
-#pragma unroll
-  for (int i = 0; i < 32; ++i) v[i] = cscale(v[i], mask_sc[G::fky(t, i) * W + G::fkx(t, i)]);
+  mul_real_table<W>(v, mask_sc);
   WinFFT<W>::inverse(v, xbuf, tw1, tw2);
   // all reads of this window finished before the first barrier of forward()
 #pragma unroll
-  for (int i = 0; i < 32; ++i) win[G::ry(t) * W + G::rx(t, i)] = v[i];
+  for (int i = 0; i < 32; ++i) win[G::ry(t) * W + G::rx(t, i)] = wget(v, i);
 }
 
 // ------------------------------------------------------------------ deterministic scatter
@@ -1246,21 +1287,24 @@ __global__ void __launch_bounds__(Geo<W>::T) probe_final_kernel(const float2* __
   __syncthreads();
   const int t = threadIdx.x, p = blockIdx.x;
   const size_t WW = (size_t)W * W;
-  // chunks outer, elements inner: each chunk's 32 loads are independent and in flight
-  // together (the chunk order of every element's sum is unchanged)
-  float2 v[32];
+  // chunks outer, elements inner: each chunk's loads are independent and in flight together
+  // (the chunk order of every element's sum is unchanged)
+  Win v;
 #pragma unroll
-  for (int i = 0; i < 32; ++i) v[i] = make_float2(0.f, 0.f);
+  for (int j = 0; j < 16; ++j) v.re[j] = v.im[j] = make_float2(0.f, 0.f);
   for (int c = 0; c < nchunk; ++c) {
-    const float2* src = partial + ((size_t)c * Mp + p) * WW;
+    const float4* src = reinterpret_cast<const float4*>(partial + ((size_t)c * Mp + p) * WW) + nword(0, t);
 #pragma unroll
-    for (int i = 0; i < 32; ++i) v[i] = cadd(v[i], src[nidx<W>(i, t)]);
+    for (int j = 0; j < 16; ++j) {
+      const float4 q = src[j * 32];
+      v.re[j] = padd(v.re[j], make_float2(q.x, q.y));
+      v.im[j] = padd(v.im[j], make_float2(q.z, q.w));
+    }
   }
-#pragma unroll
-  for (int i = 0; i < 32; ++i) v[i] = cscale(v[i], mask_sc[G::fky(t, i) * W + G::fkx(t, i)]);
+  mul_real_table<W>(v, mask_sc);
   WinFFT<W>::inverse(v, xbuf, tw1, tw2);
 #pragma unroll
-  for (int i = 0; i < 32; ++i) probe_grad[(size_t)(G::ry(t) * W + G::rx(t, i)) * Mp + p] = v[i];
+  for (int i = 0; i < 32; ++i) probe_grad[(size_t)(G::ry(t) * W + G::rx(t, i)) * Mp + p] = wget(v, i);
 }
 
 // ------------------------------------------------------------------ scalars
@@ -1330,23 +1374,23 @@ __global__ void __launch_bounds__(Geo<W>::T) fft2_batch_kernel(const float2* __r
   const size_t WW = (size_t)W * W;
   const float2* src = in + (size_t)blockIdx.x * WW;
   float2* dst = out + (size_t)blockIdx.x * WW;
-  float2 v[32];
+  Win v;
   const int h = shift ? W / 2 : 0;
   if (!inverse) {
 #pragma unroll
-    for (int i = 0; i < 32; ++i) v[i] = src[G::ry(t) * W + G::rx(t, i)];
+    for (int i = 0; i < 32; ++i) wset(v, i, src[G::ry(t) * W + G::rx(t, i)]);
     WinFFT<W>::forward(v, xbuf, tw1, tw2);
 #pragma unroll
     for (int i = 0; i < 32; ++i)
-      dst[((G::fky(t, i) + h) & (W - 1)) * W + ((G::fkx(t, i) + h) & (W - 1))] = v[i];
+      dst[((G::fky(t, i) + h) & (W - 1)) * W + ((G::fkx(t, i) + h) & (W - 1))] = wget(v, i);
   } else {
     const float inv = 1.0f / (float)WW;
 #pragma unroll
     for (int i = 0; i < 32; ++i)
-      v[i] = cscale(src[((G::fky(t, i) + h) & (W - 1)) * W + ((G::fkx(t, i) + h) & (W - 1))], inv);
+      wset(v, i, cscale(src[((G::fky(t, i) + h) & (W - 1)) * W + ((G::fkx(t, i) + h) & (W - 1))], inv));
     WinFFT<W>::inverse(v, xbuf, tw1, tw2);
 #pragma unroll
-    for (int i = 0; i < 32; ++i) dst[G::ry(t) * W + G::rx(t, i)] = v[i];
+    for (int i = 0; i < 32; ++i) dst[G::ry(t) * W + G::rx(t, i)] = wget(v, i);
   }
 }
 
@@ -1375,26 +1419,26 @@ __global__ void __launch_bounds__(Geo<W>::T) prop_step_kernel(const float2* in, 
   const float2* src = in + (size_t)blockIdx.x * WW;
   float2* dst = out + (size_t)blockIdx.x * WW;
   const float2* P = tab + (size_t)(blockIdx.x / nper) * tab_stride;
-  float2 v[32];
+  Win v;
 #pragma unroll
-  for (int i = 0; i < 32; ++i) v[i] = src[G::ry(t) * W + G::rx(t, i)];
+  for (int i = 0; i < 32; ++i) wset(v, i, src[G::ry(t) * W + G::rx(t, i)]);
   WinFFT<W>::forward(v, xbuf, tw1, tw2);
+  if (rtab) mul_real_table<W>(v, rtab);   // a real table (the band-limit mask)
+  else mul_table<W>(v, P, conj != 0);
+  if (!rtab && gout) {                    // the product spectrum
 #pragma unroll
-  for (int i = 0; i < 32; ++i) {
-    const int k = G::fky(t, i) * W + G::fkx(t, i);
-    if (rtab) {   // a real table (the band-limit mask)
-      v[i] = cscale(cscale(v[i], rtab[k]), scale);
-    } else {
-      const float2 pk = P[k];
-      const float2 prod = conj ? cmulc(v[i], pk) : cmul(v[i], pk);
-      if (gout) gout[(size_t)blockIdx.x * WW + k] = cscale(prod, gscale);   // the product spectrum
-      v[i] = cscale(prod, scale);
-    }
+    for (int i = 0; i < 32; ++i)
+      gout[(size_t)blockIdx.x * WW + G::fky(t, i) * W + G::fkx(t, i)] = cscale(wget(v, i), gscale);
   }
-  __syncthreads();   // the inverse reuses the exchange buffer
+  const float2 sc = pdup(scale);
+#pragma unroll
+  for (int j = 0; j < 16; ++j) {
+    v.re[j] = pmul(v.re[j], sc);
+    v.im[j] = pmul(v.im[j], sc);
+  }
   WinFFT<W>::inverse(v, xbuf, tw1, tw2);
 #pragma unroll
-  for (int i = 0; i < 32; ++i) dst[G::ry(t) * W + G::rx(t, i)] = v[i];
+  for (int i = 0; i < 32; ++i) dst[G::ry(t) * W + G::rx(t, i)] = wget(v, i);
 }
 
 // One forward multislice step of a batch of windows (multislice_core.py:61-80) in one pass:
@@ -1423,26 +1467,30 @@ __global__ void __launch_bounds__(Geo<W>::T) fwd_prop_kernel(const float2* __res
   float2* st = stack + (((size_t)b * Z + z) * nm + pm) * WW;
   const float2* o = ob + (((size_t)b * Z + z) * Mo + m) * WW;
   const float2* P = tab + (size_t)b * tab_stride;
-  float2 v[32];
+  Win v;
 #pragma unroll
   for (int i = 0; i < 32; ++i) {
     const int u = G::ry(t) * W + G::rx(t, i);
     const float2 in = src[u];
     st[u] = cconj(in);
-    v[i] = cmul(in, o[u]);
+    wset(v, i, cmul(in, o[u]));
   }
   WinFFT<W>::forward(v, xbuf, tw1, tw2);
+  if (spec_out) {   // FFT(in O), kept for the inside-tilt gradient
 #pragma unroll
-  for (int i = 0; i < 32; ++i) {
-    const int k = G::fky(t, i) * W + G::fkx(t, i);
-    if (spec_out) spec_out[(size_t)wi * WW + k] = v[i];   // FFT(in O), kept for the inside-tilt gradient
-    v[i] = cscale(cmul(v[i], P[k]), scale);
+    for (int i = 0; i < 32; ++i) spec_out[(size_t)wi * WW + G::fky(t, i) * W + G::fkx(t, i)] = wget(v, i);
   }
-  __syncthreads();   // the inverse reuses the exchange buffer
+  mul_table<W>(v, P, false);
+  const float2 sc = pdup(scale);
+#pragma unroll
+  for (int j = 0; j < 16; ++j) {
+    v.re[j] = pmul(v.re[j], sc);
+    v.im[j] = pmul(v.im[j], sc);
+  }
   WinFFT<W>::inverse(v, xbuf, tw1, tw2);
   float2* dst = psi + (size_t)wi * WW;
 #pragma unroll
-  for (int i = 0; i < 32; ++i) dst[G::ry(t) * W + G::rx(t, i)] = v[i];
+  for (int i = 0; i < 32; ++i) dst[G::ry(t) * W + G::rx(t, i)] = wget(v, i);
 }
 
 }  // namespace pty

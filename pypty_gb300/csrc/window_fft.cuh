@@ -3,21 +3,51 @@
 // Every thread owns 32 complex values. A 2D transform is three register rounds separated
 // by two exchanges through shared memory:
 //
-//   round 1  thread (y, n2), n2 < A=W/32 : 32-point DFT along x over x = A*n1 + n2
-//   round 2  thread (k1, m2), m2 < Bq    : twiddle w_W^(k1*n2), A-point DFT over n2 (finishes
+//   round 1  lane (m1, n2) of warp m2, n2 < A=W/32: 32-point DFT along x over x = A*n1 + n2
+//            of row y = Bq*m1 + m2
+//   round 2  lane k1 of warp m2 < Bq : twiddle w_W^(k1*n2), A-point DFT over n2 (finishes
 //            kx = k1 + 32*k2), C-point DFT along y over y = Bq*m1 + m2, twiddle w_W^(j1*m2)
-//   round 3  thread (j1, g), g < S3      : Bq-point DFT over m2 (finishes ky = j1 + C*j2),
+//   round 3  thread (j1, g), g < S3  : Bq-point DFT over m2 (finishes ky = j1 + C*j2),
 //            the thread holds kx = g + S3*q
 //
-// with C = 32/A and Bq = W/C. The forward transform runs rounds 1-2-3 and leaves the
-// spectrum in the "frequency layout"; the inverse runs 3-2-1 with conjugate twiddles and
-// leaves the window in the "real layout" (round-1 ownership). Element-wise work (object
+// with C = 32/A and Bq = W/C (the number of warps). The forward transform runs rounds 1-2-3 and
+// leaves the spectrum in the "frequency layout"; the inverse runs 3-2-1 with conjugate twiddles
+// and leaves the window in the "real layout" (round-1 ownership). Element-wise work (object
 // slice, propagator, masks, loss) happens directly in those layouts, so a multislice step
 // is FFT -> multiply -> IFFT without any extra data movement.
 //
-// Shared-memory exchanges use XOR swizzles chosen so that every half-warp of 8-byte accesses
-// touches 16 distinct bank pairs and every quarter-warp of round 1's 16-byte accesses 8 distinct
-// bank quads (no bank conflicts) for both W.
+// Synchronisation. Warp m2 owns the rows y = m2 (mod Bq) in round 1 and the residue m2 in round
+// 2, so the exchange between rounds 1 and 2 is a 32 x 32 transpose inside each warp, through the
+// warp's own 8 KB part of the exchange buffer, ordered by __syncwarp alone. In the exchange
+// between rounds 2 and 3 a warp stores only to its own part as well (rows m2*C + j1 of the
+// buffer); what crosses warps are round 3's loads, and the inverse's round 3 stores to the very
+// addresses that its thread loaded. So one FFT -> multiply -> IFFT step has two block barriers
+// (before the forward's cross-warp loads and after the inverse's cross-warp stores); outside
+// them each warp runs on its own, and its operand waits, stores and barriers of one warp overlap
+// the arithmetic of the others. A thread's stores in the forward's first exchange go where only
+// it has loaded since the last block barrier, so a transform may follow another without a
+// barrier; code that uses the buffer otherwise in between puts a block barrier before the next
+// transform.
+//
+// Packed arithmetic. The window is held as 16 packs of two values, real and imaginary parts
+// apart (struct Win), and nearly all of the arithmetic is two-wide (add/mul/fma.f32x2): the
+// kernels are bound by instruction issue, and a packed instruction does two lanes' work in one
+// issue slot. The two halves of a pack go through the same butterflies: round 1 packs the even
+// and odd x of a 16-point DFT each (a scalar radix-2 stage joins them), round 2 packs
+// neighbouring n2, round 3 packs kx and kx + W/2. The exchanges store 16-byte words of real and
+// imaginary packs, so that loads give packs without register moves.
+//
+// Shared-memory exchanges are free of bank conflicts for both W: the transpose inside a warp
+// keeps real and imaginary parts in two planes of 32 rows (k1) x 8 words of 16 bytes, words
+// XOR-swizzled by k1; the cross-warp exchange has rows of W/2 words read and written
+// contiguously.
+//
+// What bounds it: the FP32 pipe and shared-memory bandwidth by turns (about 1300 FP32 lane
+// operations per thread and 256 wavefronts per warp for a 128 x 128 transform, each close to half
+// of the measured time, and with one window per SM the two overlap only where warps run apart).
+// Against scalar arithmetic with four block barriers per transform: 1500 128-px windows,
+// transform and store, 118 -> 105 us; a 256-px 24-slice call 120 -> 100 ms; the fused 128-px
+// kernel executes 21 % fewer instructions (524 M -> 416 M per 192 blocks).
 #pragma once
 #include <cuda_runtime.h>
 #include <cstdint>
@@ -159,24 +189,182 @@ struct Geo {
   static constexpr int MINB = W == 64 ? 4 : 1;   // resident blocks per SM the kernels aim for
 
   // real layout: element i of thread t is pixel (y, x)
-  static __device__ __forceinline__ int ry(int t) { return t / A; }
+  static __device__ __forceinline__ int ry(int t) { return Bq * ((t % 32) / A) + t / 32; }
   static __device__ __forceinline__ int rx(int t, int i) { return A * i + (t % A); }
-  // frequency layout: element i of thread t is frequency (ky, kx) (unshifted FFT index)
-  static __device__ __forceinline__ int fky(int t, int i) { return (t / S3) + C * (i % Bq); }
-  static __device__ __forceinline__ int fkx(int t, int i) { return (t % S3) + S3 * (i / Bq); }
+  // frequency layout: element i of thread t is frequency (ky, kx) (unshifted FFT index); the
+  // elements 2p and 2p + 1 of a pack are W/2 apart in kx
+  static __device__ __forceinline__ int fky(int t, int i) { return (t / S3) + C * ((i >> 1) % Bq); }
+  static __device__ __forceinline__ int fkx(int t, int i) {
+    return (t % S3) + S3 * ((i >> 1) / Bq) + (W / 2) * (i & 1);
+  }
 };
 
-// Twiddle tables (built once per launch into shared memory from a global copy):
-//   tw1[n2*32 + (k1 ^ n2)] = w_W^(k1*n2),  tw2[m2*C + j1] = w_W^(j1*m2),  w_W = exp(-2 pi i/W)
-// The x twiddle w_W^(k1*n2) between the 32-point and the A-point DFT along x is applied in round
-// 2, where a thread holds one k1 and every n2: A - 1 distinct factors per thread (A - 1 table
-// reads, C * (A - 1) multiplies) instead of 31 reads and multiplies per thread in round 1.
+// ------------------------------------------------------------------ packed pairs
+// Two-wide FP32 arithmetic on the halves of a float2 (one issue slot per instruction).
+__device__ __forceinline__ float2 padd(float2 a, float2 b) {
+  float2 d;
+  asm("{.reg .b64 ra, rb, rd; mov.b64 ra, {%2, %3}; mov.b64 rb, {%4, %5}; add.rn.f32x2 rd, ra, rb; mov.b64 {%0, %1}, rd;}"
+      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+}
+__device__ __forceinline__ float2 psub(float2 a, float2 b) {
+  float2 d;
+  asm("{.reg .b64 ra, rb, rd; mov.b64 ra, {%2, %3}; mov.b64 rb, {%4, %5}; sub.rn.f32x2 rd, ra, rb; mov.b64 {%0, %1}, rd;}"
+      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+}
+__device__ __forceinline__ float2 pmul(float2 a, float2 b) {
+  float2 d;
+  asm("{.reg .b64 ra, rb, rd; mov.b64 ra, {%2, %3}; mov.b64 rb, {%4, %5}; mul.rn.f32x2 rd, ra, rb; mov.b64 {%0, %1}, rd;}"
+      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+}
+__device__ __forceinline__ float2 pfma(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("{.reg .b64 ra, rb, rc, rd; mov.b64 ra, {%2, %3}; mov.b64 rb, {%4, %5}; mov.b64 rc, {%6, %7}; "
+      "fma.rn.f32x2 rd, ra, rb, rc; mov.b64 {%0, %1}, rd;}"
+      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return d;
+}
+__device__ __forceinline__ float2 pneg(float2 a) { return make_float2(-a.x, -a.y); }
+__device__ __forceinline__ float2 pdup(float a) { return make_float2(a, a); }
+
+// (re, im) *= w for packs; nwy = -w_y, so that both products fuse
+__device__ __forceinline__ void pcmul(float2& re, float2& im, float2 wx, float2 wy, float2 nwy) {
+  const float2 r = pfma(im, nwy, pmul(re, wx));
+  im = pfma(re, wy, pmul(im, wx));
+  re = r;
+}
+
+// A window's 32 values of one thread: pack p holds elements 2p and 2p + 1, real parts and
+// imaginary parts apart.
+struct Win {
+  float2 re[16], im[16];
+};
+__device__ __forceinline__ float2 wget(const Win& v, int i) {
+  return (i & 1) ? make_float2(v.re[i >> 1].y, v.im[i >> 1].y) : make_float2(v.re[i >> 1].x, v.im[i >> 1].x);
+}
+__device__ __forceinline__ void wset(Win& v, int i, float2 a) {
+  if (i & 1) {
+    v.re[i >> 1].y = a.x;
+    v.im[i >> 1].y = a.y;
+  } else {
+    v.re[i >> 1].x = a.x;
+    v.im[i >> 1].x = a.y;
+  }
+}
+
+// In-register DFTs of packs: both halves transform alike. Radix 4 as DFT<N, SIGN> above, with
+// the values re/im[OFF + STRIDE*i], i < N, written back in natural order.
+template <int N, int E, int SIGN>
+__device__ __forceinline__ void ptw(float2& re, float2& im) {
+  static_assert(32 % N == 0, "twiddle table covers N | 32");
+  constexpr int m = ((E % N) * (32 / N)) & 31;
+  if constexpr (m == 0) {
+  } else if constexpr (m == 8 || m == 24) {   // +-i
+    constexpr bool plus = (m == 8) == (SIGN > 0);
+    const float2 r = re;
+    re = plus ? pneg(im) : im;
+    im = plus ? r : pneg(r);
+  } else if constexpr (m == 16) {
+    re = pneg(re);
+    im = pneg(im);
+  } else if constexpr (m % 4 == 0) {          // odd multiples of pi/4
+    constexpr float h = 7.071067691e-01f;
+    constexpr float c = kcos32(m) > 0 ? h : -h;
+    constexpr float s = (SIGN > 0 ? 1.0f : -1.0f) * (ksin32(m) > 0 ? h : -h);
+    constexpr bool same = (c > 0) == (s > 0);
+    const float2 u = same ? psub(re, im) : padd(re, im);
+    const float2 w = same ? padd(im, re) : psub(im, re);
+    re = pmul(u, pdup(c));
+    im = pmul(w, pdup(c));
+  } else {
+    constexpr float c = kcos32(m);
+    constexpr float s = (SIGN > 0 ? 1.0f : -1.0f) * ksin32(m);
+    pcmul(re, im, pdup(c), pdup(s), pdup(-s));
+  }
+}
+
+template <int SIGN>
+__device__ __forceinline__ void pbfly4(float2& r0, float2& i0, float2& r1, float2& i1, float2& r2, float2& i2,
+                                       float2& r3, float2& i3) {
+  const float2 ur0 = padd(r0, r2), ui0 = padd(i0, i2), ur1 = psub(r0, r2), ui1 = psub(i0, i2);
+  const float2 ur2 = padd(r1, r3), ui2 = padd(i1, i3), dr = psub(r1, r3), di = psub(i1, i3);
+  r0 = padd(ur0, ur2);
+  i0 = padd(ui0, ui2);
+  r2 = psub(ur0, ur2);
+  i2 = psub(ui0, ui2);
+  // u3 = d * (SIGN * i) = SIGN * (-di, dr)
+  r1 = SIGN > 0 ? psub(ur1, di) : padd(ur1, di);
+  i1 = SIGN > 0 ? padd(ui1, dr) : psub(ui1, dr);
+  r3 = SIGN > 0 ? padd(ur1, di) : psub(ur1, di);
+  i3 = SIGN > 0 ? psub(ui1, dr) : padd(ui1, dr);
+}
+
+template <int N, int SIGN>
+struct PDFT {
+  template <int STRIDE, int OFF>
+  static __device__ __forceinline__ void run(float2 (&re)[16], float2 (&im)[16]) {
+    if constexpr (N == 1) {
+    } else if constexpr (N == 2) {
+      const float2 ar = re[OFF], ai = im[OFF], br = re[OFF + STRIDE], bi = im[OFF + STRIDE];
+      re[OFF] = padd(ar, br);
+      im[OFF] = padd(ai, bi);
+      re[OFF + STRIDE] = psub(ar, br);
+      im[OFF + STRIDE] = psub(ai, bi);
+    } else if constexpr (N == 4) {
+      pbfly4<SIGN>(re[OFF], im[OFF], re[OFF + STRIDE], im[OFF + STRIDE], re[OFF + 2 * STRIDE], im[OFF + 2 * STRIDE],
+                   re[OFF + 3 * STRIDE], im[OFF + 3 * STRIDE]);
+    } else {
+      constexpr int M = N / 4;
+      PDFT<M, SIGN>::template run<4 * STRIDE, OFF>(re, im);
+      PDFT<M, SIGN>::template run<4 * STRIDE, OFF + STRIDE>(re, im);
+      PDFT<M, SIGN>::template run<4 * STRIDE, OFF + 2 * STRIDE>(re, im);
+      PDFT<M, SIGN>::template run<4 * STRIDE, OFF + 3 * STRIDE>(re, im);
+      float2 outr[N], outi[N];
+      static_for<0, M>([&](auto KK) {
+        constexpr int k = decltype(KK)::value;
+        float2 r0 = re[OFF + STRIDE * (4 * k)], i0 = im[OFF + STRIDE * (4 * k)];
+        float2 r1 = re[OFF + STRIDE * (4 * k + 1)], i1 = im[OFF + STRIDE * (4 * k + 1)];
+        float2 r2 = re[OFF + STRIDE * (4 * k + 2)], i2 = im[OFF + STRIDE * (4 * k + 2)];
+        float2 r3 = re[OFF + STRIDE * (4 * k + 3)], i3 = im[OFF + STRIDE * (4 * k + 3)];
+        ptw<N, 1 * k, SIGN>(r1, i1);
+        ptw<N, 2 * k, SIGN>(r2, i2);
+        ptw<N, 3 * k, SIGN>(r3, i3);
+        pbfly4<SIGN>(r0, i0, r1, i1, r2, i2, r3, i3);
+        outr[k] = r0, outi[k] = i0;
+        outr[k + M] = r1, outi[k + M] = i1;
+        outr[k + 2 * M] = r2, outi[k + 2 * M] = i2;
+        outr[k + 3 * M] = r3, outi[k + 3 * M] = i3;
+      });
+#pragma unroll
+      for (int i = 0; i < N; ++i) {
+        re[OFF + STRIDE * i] = outr[i];
+        im[OFF + STRIDE * i] = outi[i];
+      }
+    }
+  }
+};
+
+// Twiddle tables, in global memory (twiddle_entry): w_W^(k1*n2) at n2*32 + k1, then w_W^(j1*m2)
+// at m2*C + j1, w_W = exp(-2 pi i/W); in shared memory (load_twiddles) as the packed arithmetic
+// reads them: tw1 the cosines [k1][n2] then the sines [k1][n2], tw2 (cos, cos, sin, sin) per
+// entry. The x twiddle w_W^(k1*n2) between the 32-point and the A-point DFT along x is applied
+// in round 2, where a thread holds one k1 and every n2.
 template <int W>
 __device__ __forceinline__ void load_twiddles(float2* s_tw1, float2* s_tw2, const float2* g_tw) {
   using G = Geo<W>;
+  float* t1 = reinterpret_cast<float*>(s_tw1);
+  float4* t2 = reinterpret_cast<float4*>(s_tw2);
   for (int i = threadIdx.x; i < G::TW1 + G::TW2; i += blockDim.x) {
-    float2 w = g_tw[i];
-    if (i < G::TW1) s_tw1[i] = w; else s_tw2[i - G::TW1] = w;
+    const float2 w = g_tw[i];
+    if (i < G::TW1) {
+      const int n2 = i / 32, k1 = i % 32;
+      t1[k1 * G::A + n2] = w.x;
+      t1[G::TW1 + k1 * G::A + n2] = w.y;
+    } else {
+      t2[i - G::TW1] = make_float4(w.x, w.x, w.y, w.y);
+    }
   }
 }
 
@@ -184,182 +372,228 @@ template <int W>
 struct WinFFT {
   using G = Geo<W>;
   static constexpr int A = G::A, C = G::C, Bq = G::Bq, Q = G::Q, S3 = G::S3;
+  static constexpr int WPART = 1024;   // float2 of the exchange buffer that a warp owns
+  static constexpr int PLANE = 1024;   // floats of one plane (real or imaginary) of the warp's transpose
+  static constexpr int H = W / 2;      // words of a row of the cross-warp exchange
 
-  // the XOR masks are even, so a row's elements 2j and 2j+1 stay adjacent: round 1 moves them
-  // as one 16-byte word (round 2 reads single elements), conflict-free both ways
-  static __device__ __forceinline__ int x1(int r, int k1) { return r * 32 + (k1 ^ ((r & 7) << 1)); }
-  static __device__ __forceinline__ int x2(int s, int kx) { return s * W + (kx ^ ((s & 1) << 3)); }
+  // the x twiddles of this lane's k1 as packs over n2: pack h of A/2 covers n2 = 2h, 2h + 1
+  struct Tw1 {
+    float2 x[A / 2], y[A / 2];
+    __device__ __forceinline__ Tw1(const float2* tw1, int k1) {
+      const float2* t = tw1 + k1 * (A / 2);
+#pragma unroll
+      for (int h = 0; h < A / 2; ++h) {
+        x[h] = t[h];
+        y[h] = t[G::TW1 / 2 + h];
+      }
+    }
+  };
 
   // real layout -> frequency layout, unnormalised, exp(-2 pi i ...) kernel
-  static __device__ __forceinline__ void forward(float2 (&v)[32], float2* xbuf,
-                                                 const float2* tw1, const float2* tw2) {
-    forward_round1(v, tw1);
-    forward_rest(v, xbuf, tw1, tw2, [] {});
-  }
-
-  // The forward transform in two parts, so that a caller can overlap work that must finish
-  // before the exchange buffer is overwritten (a cluster barrier, a pending copy) with the
-  // register-only first round. forward_round1 touches no shared memory besides the twiddles;
-  // forward_rest calls after_first_sync() right after its first barrier, when every thread of
-  // the block has finished everything it did before forward_rest.
-  static __device__ __forceinline__ void forward_round1(float2 (&v)[32], const float2* tw1) {
-    (void)tw1;   // the x twiddle is applied in round 2
-    DFT<32, -1>::template run<32, 1, 0>(v);
-  }
-
-  template <typename AfterSync>
-  static __device__ __forceinline__ void forward_rest(float2 (&v)[32], float2* xbuf, const float2* tw1,
-                                                     const float2* tw2, AfterSync&& after_first_sync) {
-    const int t = threadIdx.x;
-    __syncthreads();
-    after_first_sync();
-#pragma unroll
-    for (int j = 0; j < 16; ++j)
-      reinterpret_cast<float4*>(xbuf)[x1(t, 2 * j) >> 1] =
-          make_float4(v[2 * j].x, v[2 * j].y, v[2 * j + 1].x, v[2 * j + 1].y);
-    __syncthreads();
-    // ---- round 2
+  static __device__ __forceinline__ void forward(Win& v, float2* xbuf, const float2* tw1, const float2* tw2) {
+    const int t = threadIdx.x, lane = t % 32, m2 = t / 32;   // lane: round 1's row, round 2's k1
+    float* xw = reinterpret_cast<float*>(xbuf + m2 * WPART);
+    float4* x4 = reinterpret_cast<float4*>(xbuf);
+    // ---- round 1: 16-point DFTs of the even and odd x, then X_k, X_{k+16} = E_k +- w_32^k O_k
+    PDFT<16, -1>::template run<1, 0>(v.re, v.im);
+    static_for<0, 16>([&](auto KK) {
+      constexpr int k = decltype(KK)::value;
+      const float2 o = tw<32, k, -1>(make_float2(v.re[k].y, v.im[k].y));
+      const float2 e = make_float2(v.re[k].x, v.im[k].x);
+      const float2 a = cadd(e, o), b = csub(e, o);
+      // row k1, word (lane / 4) ^ (k1 & 7); rows k and k + 16 share the swizzle
+      float* d = xw + k * 32 + ((((lane >> 2) ^ (k & 7)) << 2) | (lane & 3));
+      d[0] = a.x;
+      d[PLANE] = a.y;
+      d[16 * 32] = b.x;
+      d[16 * 32 + PLANE] = b.y;
+    });
+    __syncwarp();
+    // ---- round 2: word c of row k1 = lane holds local rows 4c .. 4c + 3 (row m1*A + n2)
     {
-      const int k1 = t % 32, m2 = t / 32;
+      const float4* p4 = reinterpret_cast<const float4*>(xw) + lane * 8;
 #pragma unroll
-      for (int m1 = 0; m1 < C; ++m1)
-#pragma unroll
-        for (int n2 = 0; n2 < A; ++n2) v[m1 * A + n2] = xbuf[x1((Bq * m1 + m2) * A + n2, k1)];
-      {   // x twiddle w_W^(k1*n2): this thread's k1 is fixed
-        float2 w[A];
-#pragma unroll
-        for (int n2 = 1; n2 < A; ++n2) w[n2] = tw1[n2 * 32 + (k1 ^ n2)];
-#pragma unroll
-        for (int m1 = 0; m1 < C; ++m1)
-#pragma unroll
-          for (int n2 = 1; n2 < A; ++n2) v[m1 * A + n2] = cmul(v[m1 * A + n2], w[n2]);
+      for (int c = 0; c < 8; ++c) {
+        const float4 r = p4[c ^ (lane & 7)], i = p4[(c ^ (lane & 7)) + PLANE / 4];
+        v.re[2 * c] = make_float2(r.x, r.y);
+        v.re[2 * c + 1] = make_float2(r.z, r.w);
+        v.im[2 * c] = make_float2(i.x, i.y);
+        v.im[2 * c + 1] = make_float2(i.z, i.w);
       }
-      static_for<0, C>([&](auto M1) { DFT<A, -1>::template run<32, 1, decltype(M1)::value * A>(v); });
-      static_for<0, A>([&](auto K2) { DFT<C, -1>::template run<32, A, decltype(K2)::value>(v); });
-      if (m2 != 0) {
+    }
+    {   // x twiddle w_W^(k1*n2): this thread's k1 is fixed
+      const Tw1 w(tw1, lane);
 #pragma unroll
-        for (int j1 = 1; j1 < C; ++j1) {
-          float2 w = tw2[m2 * C + j1];
+      for (int h = 0; h < A / 2; ++h) {
+        const float2 ny = pneg(w.y[h]);
 #pragma unroll
-          for (int k2 = 0; k2 < A; ++k2) v[j1 * A + k2] = cmul(v[j1 * A + k2], w);
-        }
+        for (int m1 = 0; m1 < C; ++m1) pcmul(v.re[m1 * (A / 2) + h], v.im[m1 * (A / 2) + h], w.x[h], w.y[h], ny);
       }
-      __syncthreads();
+    }
+    static_for<0, A / 2>([&](auto HH) { PDFT<C, -1>::template run<A / 2, decltype(HH)::value>(v.re, v.im); });
+    if (m2 != 0) {
+      const float4* t2 = reinterpret_cast<const float4*>(tw2) + m2 * C;
 #pragma unroll
-      for (int j1 = 0; j1 < C; ++j1)
+      for (int j1 = 1; j1 < C; ++j1) {
+        const float4 w = t2[j1];
+        const float2 ws = make_float2(w.z, w.w), ns = pneg(ws);
 #pragma unroll
-        for (int k2 = 0; k2 < A; ++k2) xbuf[x2(m2 * C + j1, k1 + 32 * k2)] = v[j1 * A + k2];
+        for (int h = 0; h < A / 2; ++h)
+          pcmul(v.re[j1 * (A / 2) + h], v.im[j1 * (A / 2) + h], make_float2(w.x, w.y), ws, ns);
+      }
+    }
+    __syncwarp();   // the warp has read its transpose
+    // A-point DFT over n2, joining the halves of the packs; kx and kx + W/2 leave as one word
+    // (re, re', im, im')
+#pragma unroll
+    for (int j1 = 0; j1 < C; ++j1) {
+      float4* row = x4 + (m2 * C + j1) * H + lane;
+      if constexpr (A == 2) {
+        const float2 r = v.re[j1], i = v.im[j1];
+        row[0] = make_float4(r.x + r.y, r.x - r.y, i.x + i.y, i.x - i.y);
+      } else {
+        const float2 ur = padd(v.re[2 * j1], v.re[2 * j1 + 1]), ui = padd(v.im[2 * j1], v.im[2 * j1 + 1]);
+        const float2 dr = psub(v.re[2 * j1], v.re[2 * j1 + 1]), di = psub(v.im[2 * j1], v.im[2 * j1 + 1]);
+        row[0] = make_float4(ur.x + ur.y, ur.x - ur.y, ui.x + ui.y, ui.x - ui.y);         // k2 = 0, 2
+        row[32] = make_float4(dr.x + di.y, dr.x - di.y, di.x - dr.y, di.x + dr.y);        // k2 = 1, 3
+      }
     }
     __syncthreads();
     // ---- round 3
     {
       const int g = t % S3, j1 = t / S3;
+      const float4* col = x4 + j1 * H + g;
 #pragma unroll
-      for (int q = 0; q < Q; ++q)
+      for (int q = 0; q < Q / 2; ++q)
 #pragma unroll
-        for (int m2 = 0; m2 < Bq; ++m2) v[q * Bq + m2] = xbuf[x2(m2 * C + j1, g + S3 * q)];
-      static_for<0, Q>([&](auto QQ) { DFT<Bq, -1>::template run<32, 1, decltype(QQ)::value * Bq>(v); });
+        for (int r = 0; r < Bq; ++r) {
+          const float4 w = col[r * C * H + S3 * q];
+          v.re[q * Bq + r] = make_float2(w.x, w.y);
+          v.im[q * Bq + r] = make_float2(w.z, w.w);
+        }
+      static_for<0, Q / 2>([&](auto QQ) { PDFT<Bq, -1>::template run<1, decltype(QQ)::value * Bq>(v.re, v.im); });
     }
   }
 
   // frequency layout -> real layout, unnormalised, exp(+2 pi i ...) kernel (no 1/W^2)
-  static __device__ __forceinline__ void inverse(float2 (&v)[32], float2* xbuf,
-                                                 const float2* tw1, const float2* tw2) {
+  static __device__ __forceinline__ void inverse(Win& v, float2* xbuf, const float2* tw1, const float2* tw2) {
     inverse_head(v, xbuf, tw1, tw2);
-    inverse_tail(v, tw1);
+    inverse_tail(v);
   }
 
   // The register-only end of the inverse transform (round 1): callers that reuse xbuf may
-  // run inverse_head (everything up to the last xbuf read), synchronise, refill xbuf
-  // asynchronously, and then run inverse_tail while the copy is in flight.
-  static __device__ __forceinline__ void inverse_tail(float2 (&v)[32], const float2* tw1) {
-    (void)tw1;   // the conjugate x twiddle was applied in round 2 of inverse_head
-    DFT<32, +1>::template run<32, 1, 0>(v);
-  }
+  // run inverse_head (everything up to the last xbuf read), __syncwarp, refill the warp's part
+  // of xbuf asynchronously, and then run inverse_tail while the copy is in flight.
+  static __device__ __forceinline__ void inverse_tail(Win& v) { PDFT<16, +1>::template run<1, 0>(v.re, v.im); }
 
-  // inverse() without its register-only tail: after it returns (and a barrier), xbuf is free.
-  static __device__ __forceinline__ void inverse_head(float2 (&v)[32], float2* xbuf,
-                                                      const float2* tw1, const float2* tw2) {
-    const int t = threadIdx.x;
+  // inverse() without its register-only tail
+  static __device__ __forceinline__ void inverse_head(Win& v, float2* xbuf, const float2* tw1, const float2* tw2) {
+    const int t = threadIdx.x, lane = t % 32, m2 = t / 32;
+    float* xw = reinterpret_cast<float*>(xbuf + m2 * WPART);
+    float4* x4 = reinterpret_cast<float4*>(xbuf);
     {
       const int g = t % S3, j1 = t / S3;
-      static_for<0, Q>([&](auto QQ) { DFT<Bq, +1>::template run<32, 1, decltype(QQ)::value * Bq>(v); });
-      __syncthreads();
+      static_for<0, Q / 2>([&](auto QQ) { PDFT<Bq, +1>::template run<1, decltype(QQ)::value * Bq>(v.re, v.im); });
+      // the addresses that this thread loaded in the forward's round 3: no barrier between
+      float4* col = x4 + j1 * H + g;
 #pragma unroll
-      for (int q = 0; q < Q; ++q)
+      for (int q = 0; q < Q / 2; ++q)
 #pragma unroll
-        for (int m2 = 0; m2 < Bq; ++m2) xbuf[x2(m2 * C + j1, g + S3 * q)] = v[q * Bq + m2];
+        for (int r = 0; r < Bq; ++r)
+          col[r * C * H + S3 * q] =
+              make_float4(v.re[q * Bq + r].x, v.re[q * Bq + r].y, v.im[q * Bq + r].x, v.im[q * Bq + r].y);
     }
     __syncthreads();
+#pragma unroll
+    for (int j1 = 0; j1 < C; ++j1) {
+      const float4* row = x4 + (m2 * C + j1) * H + lane;
+      if constexpr (A == 2) {
+        const float4 a = row[0];
+        v.re[j1] = make_float2(a.x + a.y, a.x - a.y);
+        v.im[j1] = make_float2(a.z + a.w, a.z - a.w);
+      } else {
+        const float4 a = row[0], b = row[32];   // X0, X2 and X1, X3
+        const float2 ur = make_float2(a.x + a.y, a.x - a.y), ui = make_float2(a.z + a.w, a.z - a.w);
+        // (X1 + X3, i (X1 - X3))
+        const float2 sr = make_float2(b.x + b.y, b.w - b.z), si = make_float2(b.z + b.w, b.x - b.y);
+        v.re[2 * j1] = padd(ur, sr);
+        v.im[2 * j1] = padd(ui, si);
+        v.re[2 * j1 + 1] = psub(ur, sr);
+        v.im[2 * j1 + 1] = psub(ui, si);
+      }
+    }
+    if (m2 != 0) {
+      const float4* t2 = reinterpret_cast<const float4*>(tw2) + m2 * C;
+#pragma unroll
+      for (int j1 = 1; j1 < C; ++j1) {
+        const float4 w = t2[j1];
+        const float2 ws = make_float2(w.z, w.w), ns = pneg(ws);
+#pragma unroll
+        for (int h = 0; h < A / 2; ++h)
+          pcmul(v.re[j1 * (A / 2) + h], v.im[j1 * (A / 2) + h], make_float2(w.x, w.y), ns, ws);
+      }
+    }
+    static_for<0, A / 2>([&](auto HH) { PDFT<C, +1>::template run<A / 2, decltype(HH)::value>(v.re, v.im); });
+    {   // conjugate x twiddle w_W^(-k1*n2), this thread's k1 fixed
+      const Tw1 w(tw1, lane);
+#pragma unroll
+      for (int h = 0; h < A / 2; ++h) {
+        const float2 ny = pneg(w.y[h]);
+#pragma unroll
+        for (int m1 = 0; m1 < C; ++m1) pcmul(v.re[m1 * (A / 2) + h], v.im[m1 * (A / 2) + h], w.x[h], ny, w.y[h]);
+      }
+    }
+    __syncwarp();   // the warp has read its part of the cross-warp exchange
     {
-      const int k1 = t % 32, m2 = t / 32;
+      float4* p4 = reinterpret_cast<float4*>(xw) + lane * 8;
 #pragma unroll
-      for (int j1 = 0; j1 < C; ++j1)
-#pragma unroll
-        for (int k2 = 0; k2 < A; ++k2) v[j1 * A + k2] = xbuf[x2(m2 * C + j1, k1 + 32 * k2)];
-      if (m2 != 0) {
-#pragma unroll
-        for (int j1 = 1; j1 < C; ++j1) {
-          float2 w = tw2[m2 * C + j1];
-#pragma unroll
-          for (int k2 = 0; k2 < A; ++k2) v[j1 * A + k2] = cmulc(v[j1 * A + k2], w);
-        }
+      for (int c = 0; c < 8; ++c) {
+        p4[c ^ (lane & 7)] = make_float4(v.re[2 * c].x, v.re[2 * c].y, v.re[2 * c + 1].x, v.re[2 * c + 1].y);
+        p4[(c ^ (lane & 7)) + PLANE / 4] = make_float4(v.im[2 * c].x, v.im[2 * c].y, v.im[2 * c + 1].x, v.im[2 * c + 1].y);
       }
-      static_for<0, A>([&](auto K2) { DFT<C, +1>::template run<32, A, decltype(K2)::value>(v); });
-      static_for<0, C>([&](auto M1) { DFT<A, +1>::template run<32, 1, decltype(M1)::value * A>(v); });
-      {   // conjugate x twiddle w_W^(-k1*n2), this thread's k1 fixed
-        float2 w[A];
-#pragma unroll
-        for (int n2 = 1; n2 < A; ++n2) w[n2] = tw1[n2 * 32 + (k1 ^ n2)];
-#pragma unroll
-        for (int m1 = 0; m1 < C; ++m1)
-#pragma unroll
-          for (int n2 = 1; n2 < A; ++n2) v[m1 * A + n2] = cmulc(v[m1 * A + n2], w[n2]);
-      }
-      __syncthreads();
-#pragma unroll
-      for (int m1 = 0; m1 < C; ++m1)
-#pragma unroll
-        for (int n2 = 0; n2 < A; ++n2) xbuf[x1((Bq * m1 + m2) * A + n2, k1)] = v[m1 * A + n2];
     }
-    __syncthreads();
-#pragma unroll
-    for (int j = 0; j < 16; ++j) {
-      const float4 q = reinterpret_cast<const float4*>(xbuf)[x1(t, 2 * j) >> 1];
-      v[2 * j] = make_float2(q.x, q.y);
-      v[2 * j + 1] = make_float2(q.z, q.w);
-    }
+    __syncwarp();
+    static_for<0, 16>([&](auto KK) {
+      constexpr int k = decltype(KK)::value;
+      const float* d = xw + k * 32 + ((((lane >> 2) ^ (k & 7)) << 2) | (lane & 3));
+      const float2 a = make_float2(d[0], d[PLANE]), b = make_float2(d[16 * 32], d[16 * 32 + PLANE]);
+      const float2 e = cadd(a, b), o = tw<32, k, +1>(csub(a, b));
+      v.re[k] = make_float2(e.x, o.x);
+      v.im[k] = make_float2(e.y, o.y);
+    });
   }
 };
 
 // ------------------------------------------------------------------ native window layout
 // Windows that live only inside the library are stored in the order the FFT threads own
-// them: element i of thread t at float2 offset 2*((i/2)*T + t) + i%2. A thread's element
-// pair (2j, 2j+1) is one 16-byte word and a warp touches 512 contiguous bytes per access.
-// Elements i < 2j of every thread form one contiguous prefix (2j*T float2).
-template <int W>
-__device__ __forceinline__ int nidx(int i, int t) {
-  return 2 * ((i >> 1) * Geo<W>::T + t) + (i & 1);
-}
+// them, warp by warp: pack p of lane l of warp w is the 16-byte word (re, re', im, im') at word
+// w*512 + p*32 + l. A warp touches 512 contiguous bytes per access, and a warp's whole share is
+// 8 KB in one piece (its first 512*p bytes the packs below p), so each warp's operands move by
+// bulk copies of its own.
+__device__ __forceinline__ int nword(int p, int t) { return (t >> 5) * 512 + p * 32 + (t & 31); }   // in float4
 
-template <int W>
-__device__ __forceinline__ void ld_native(const float2* base, float2 (&v)[32]) {
-  const float4* p = reinterpret_cast<const float4*>(base);
-  const int t = threadIdx.x;
+__device__ __forceinline__ float4 pack4(float2 re, float2 im) { return make_float4(re.x, re.y, im.x, im.y); }
+
+__device__ __forceinline__ void ld_native(const float2* base, Win& v) {
+  const float4* p = reinterpret_cast<const float4*>(base) + nword(0, threadIdx.x);
 #pragma unroll
   for (int j = 0; j < 16; ++j) {
-    const float4 q = p[j * Geo<W>::T + t];
-    v[2 * j] = make_float2(q.x, q.y);
-    v[2 * j + 1] = make_float2(q.z, q.w);
+    const float4 q = p[j * 32];
+    v.re[j] = make_float2(q.x, q.y);
+    v.im[j] = make_float2(q.z, q.w);
   }
 }
 
-template <int W>
-__device__ __forceinline__ void st_native(float2* base, const float2 (&v)[32]) {
-  float4* p = reinterpret_cast<float4*>(base);
-  const int t = threadIdx.x;
+__device__ __forceinline__ void st_native(float2* base, const Win& v) {
+  float4* p = reinterpret_cast<float4*>(base) + nword(0, threadIdx.x);
 #pragma unroll
-  for (int j = 0; j < 16; ++j) p[j * Geo<W>::T + t] = make_float4(v[2 * j].x, v[2 * j].y, v[2 * j + 1].x, v[2 * j + 1].y);
+  for (int j = 0; j < 16; ++j) p[j * 32] = pack4(v.re[j], v.im[j]);
+}
+
+// element i of thread t of a native window
+__device__ __forceinline__ float2 native_at(const float2* base, int i, int t) {
+  const float* w = reinterpret_cast<const float*>(reinterpret_cast<const float4*>(base) + nword(i >> 1, t));
+  return make_float2(w[i & 1], w[2 + (i & 1)]);
 }
 
 // ------------------------------------------------------------------ bulk async copies
@@ -480,7 +714,7 @@ __device__ __forceinline__ float2 twiddle_entry(int i) {
   using G = Geo<W>;
   int e;
   if (i < G::TW1) {
-    int n2 = i / 32, k1 = (i % 32) ^ n2;
+    int n2 = i / 32, k1 = i % 32;
     e = (k1 * n2) % W;
   } else {
     int j = i - G::TW1, m2 = j / G::C, j1 = j % G::C;
