@@ -63,8 +63,9 @@ struct Path {
     const size_t smem = Smem<W>::bytes;
     int rc;
     if ((rc = set_smem(probe_fft_kernel<W>, smem)) || (rc = set_smem(object_windows_kernel<W>, smem)) ||
-        (rc = set_smem(fused_multislice_kernel<W, 0>, FusedSmem<W>::bytes)) ||
-        (rc = set_smem(fused_multislice_kernel<W, 1>, FusedSmem<W>::bytes)) ||
+        (rc = set_smem(fused_multislice_kernel<W, PH_WHOLE>, FusedSmem<W>::bytes)) ||
+        (rc = set_smem(fused_multislice_kernel<W, PH_FWD>, FusedSmem<W>::bytes)) ||
+        (rc = set_smem(fused_multislice_kernel<W, PH_ADJ>, FusedSmem<W>::bytes)) ||
         (rc = set_smem(grad_windows_kernel<W>, smem)) || (rc = set_smem(probe_final_kernel<W>, smem)))
       return rc;
     return PTY_OK;
@@ -160,8 +161,29 @@ struct Path {
     return cuda_status();
   }
 
-  // phase 0: the whole pass; 1: forward half (keeps the wave stack and dL/d(exit wave));
-  // 2: adjoint half
+  // One launch of the fused kernel's part PH for Bn positions, in clusters of the position's
+  // modes where its blocks exchange data.
+  template <int PH>
+  static int launch_fused(const FusedArgs& fa, int Bn, cudaStream_t st) {
+    const int nmodes = fa.Mp * fa.Mo;
+    const bool clusters = PH == PH_WHOLE || (PH == PH_ADJ && fa.Mo > 1);
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)(Bn * nmodes));
+    cfg.blockDim = dim3(T);
+    cfg.dynamicSmemBytes = FusedSmem<W>::bytes;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = clusters ? (unsigned)nmodes : 1u;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, fused_multislice_kernel<W, PH>, fa) == cudaSuccess ? PTY_OK : PTY_ERR_CUDA;
+  }
+
+  // phase 0: the whole pass; 1: forward half (keeps the wave stack, the far field and dL/dI);
+  // 2: adjoint half. The whole pass runs as its two halves where the plan says so (q.halves).
   int fused(int ib, int phase, const float2* probe, const float* measured, float* patterns) {
     const int Bn = batch_count(ib);
     const int s0 = ib * q.Bb;
@@ -177,7 +199,6 @@ struct Path {
     fa.probe_shift = p->probe_shift ? 1 : 0;
     fa.simulate = simulate ? 1 : 0;
     fa.use_edge = ta.use_edge;
-    fa.phase = phase;
     fa.loss_weight = p->loss_weight;
     fa.probe = probe;
     fa.probe_f = at<float2>(ws, q.o_probe_f);
@@ -198,29 +219,25 @@ struct Path {
     fa.stack = stack(ib);
     fa.gsum = gsum(ib);
     fa.fprobe = fprobe(ib);
-    fa.gbuf = at<float2>(ws, q.o_gbuf);
+    fa.psi = at<float2>(ws, q.o_psi + (size_t)(ib % q.nbuf) * q.s_psi);
+    fa.dldi = at<float>(ws, q.o_dldi + (size_t)(ib % q.nbuf) * q.s_dldi);
     fa.loss_part = at<double>(ws, q.o_loss_part) + 2 * (size_t)s0;
     fa.pos_part = at<double>(ws, q.o_pos_part) + 2 * (size_t)s0 * q.Mp;
     fa.sim_out = simulate ? patterns + (size_t)s0 * WW : nullptr;
     fa.err = at<int>(ws, q.o_err);
-    const int nmodes = q.Mp * q.Mo;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)(Bn * nmodes));
-    cfg.blockDim = dim3(T);
-    cfg.dynamicSmemBytes = FusedSmem<W>::bytes;
-    cfg.stream = fst;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = (unsigned)nmodes;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    prof_mark(fst, KID_FUSED);
-    const cudaError_t e = fa.phase == 0 ? cudaLaunchKernelEx(&cfg, fused_multislice_kernel<W, 0>, fa)
-                                        : cudaLaunchKernelEx(&cfg, fused_multislice_kernel<W, 1>, fa);
-    if (e != cudaSuccess) return PTY_ERR_CUDA;
-    return cuda_status();
+    prof_mark(fst, KID_FUSED);   // the halves and the loss between them are profiled as one
+    int rc;
+    if (phase == 0 && !q.halves) {
+      rc = launch_fused<PH_WHOLE>(fa, Bn, fst);
+    } else {
+      rc = PTY_OK;
+      if (phase != 2) {
+        rc = launch_fused<PH_FWD>(fa, Bn, fst);
+        if (!rc) far_field_loss_kernel<W><<<Bn, T, 0, fst>>>(fa);
+      }
+      if (!rc && phase != 1 && !simulate) rc = launch_fused<PH_ADJ>(fa, Bn, fst);
+    }
+    return rc ? rc : cuda_status();
   }
 
   int gradients(int ib) {
@@ -415,31 +432,25 @@ int run_backward(const pty_problem_t* p, const Plan& q, double* loss_sse, float2
 }
 
 // ------------------------------------------------------------------ multislice_core seams
-// Shared launch of the fused kernel on caller-given windows (phase 3 or 4).
-template <int W>
-int ms_fused(const MsPlan& q, int phase, int step_obj, int step_probe, int use_edge, void* ws, cudaStream_t st) {
-  const size_t WW = (size_t)W * W;
-  if (set_smem(fused_multislice_kernel<W, 1>, FusedSmem<W>::bytes)) return PTY_ERR_CUDA;
+// Shared launch of the fused kernel on caller-given windows: PH_FWD from given probes to the exit
+// waves, or PH_ADJ from a given dL/d(exit wave).
+template <int W, int PH>
+int ms_fused(const MsPlan& q, int step_obj, int step_probe, int use_edge, void* ws, cudaStream_t st) {
   FusedArgs fa{};
   fa.Z = q.Z;
   fa.Mp = q.Mp;
   fa.Mo = q.Mo;
-  fa.algorithm = 0;
   fa.step_obj = step_obj;
   fa.step_probe = step_probe;
-  fa.step_pos = 0;
-  fa.probe_shift = 0;
-  fa.simulate = 0;
   fa.use_edge = use_edge;
-  fa.phase = phase;
   fa.loss_weight = 1.0f;
-  fa.probe_b = phase == 3 ? at<float2>(ws, q.o_probe_b) : nullptr;
-  fa.exit_out = at<float2>(ws, q.o_gbuf);
+  fa.probe_b = PH == PH_FWD ? at<float2>(ws, q.o_probe_b) : nullptr;
+  fa.exit_out = PH == PH_FWD ? at<float2>(ws, q.o_gbuf) : nullptr;
+  fa.gbuf = PH == PH_ADJ ? at<float2>(ws, q.o_gbuf) : nullptr;
   fa.obl = at<float2>(ws, q.o_obl);
   fa.prop = at<float2>(ws, q.o_prop);
   fa.prop_edge = at<float2>(ws, q.o_prop_edge);
   fa.pyx = at<float2>(ws, q.o_pyx);
-  fa.use_sep = 0;
   fa.mask = at<float>(ws, q.o_mask);
   fa.sx = at<float>(ws, q.o_corr);     // not read without a probe shift
   fa.sy = at<float>(ws, q.o_corr);
@@ -449,26 +460,10 @@ int ms_fused(const MsPlan& q, int phase, int step_obj, int step_probe, int use_e
   fa.stack = at<float2>(ws, q.o_stack);
   fa.gsum = at<float2>(ws, q.o_gsum);
   fa.fprobe = at<float2>(ws, q.o_fprobe);
-  fa.gbuf = at<float2>(ws, q.o_gbuf);
-  fa.loss_part = at<double>(ws, q.o_parts);
-  fa.pos_part = at<double>(ws, q.o_parts) + 2 * (size_t)q.B;
   fa.err = at<int>(ws, q.o_err);
-  const int nmodes = q.Mp * q.Mo;
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3((unsigned)(q.B * nmodes));
-  cfg.blockDim = dim3(Geo<W>::T);
-  cfg.dynamicSmemBytes = FusedSmem<W>::bytes;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = (unsigned)nmodes;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
   prof_mark(st, KID_FUSED);
-  if (cudaLaunchKernelEx(&cfg, fused_multislice_kernel<W, 1>, fa) != cudaSuccess) return PTY_ERR_CUDA;
-  return cuda_status();
+  const int rc = Path<W>::template launch_fused<PH>(fa, q.B, st);
+  return rc ? rc : cuda_status();
 }
 
 template <int W>
@@ -498,7 +493,7 @@ int run_ms_forward(const MsPlan& q, const float2* probe_b, const float2* obj_b, 
   prof_mark(st, KID_LAYOUT);
   ref_to_native_kernel<W><<<q.B * q.Mp, T, 0, st>>>(probe_b, at<float2>(ws, q.o_probe_b), q.Mp, 0);
   ref_to_native_kernel<W><<<q.B * q.zm, T, 0, st>>>(obj_b, at<float2>(ws, q.o_obl), q.zm, 0);
-  if ((rc = ms_fused<W>(q, 3, 1, 0, (edge_mult > 1.0f && q.Z > 1) ? 1 : 0, ws, st))) return rc;
+  if ((rc = ms_fused<W, PH_FWD>(q, 1, 0, (edge_mult > 1.0f && q.Z > 1) ? 1 : 0, ws, st))) return rc;
   prof_mark(st, KID_LAYOUT);
   native_to_ref_kernel<W><<<q.B * q.Z * q.Mp * q.Mo, T, 0, st>>>(at<float2>(ws, q.o_stack), waves,
                                                                 q.Z * q.Mp * q.Mo, 1);
@@ -521,7 +516,7 @@ int run_ms_grads(const MsPlan& q, const float2* d_exit, const float2* waves, con
   if (step_obj)
     ref_to_native_kernel<W><<<q.B * q.Z * q.Mp * q.Mo, T, 0, st>>>(waves, at<float2>(ws, q.o_stack),
                                                                   q.Z * q.Mp * q.Mo, 1);
-  if ((rc = ms_fused<W>(q, 4, step_obj, probe_grad != nullptr, (edge_mult > 1.0f && q.Z > 1) ? 1 : 0, ws, st)))
+  if ((rc = ms_fused<W, PH_ADJ>(q, step_obj, probe_grad != nullptr, (edge_mult > 1.0f && q.Z > 1) ? 1 : 0, ws, st)))
     return rc;
   if (step_obj) {
     float2* gs = at<float2>(ws, q.o_gsum);

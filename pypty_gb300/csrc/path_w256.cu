@@ -120,7 +120,6 @@ struct Path256 {
     fa.probe_shift = p->probe_shift ? 1 : 0;
     fa.simulate = simulate ? 1 : 0;
     fa.use_edge = ta.use_edge;
-    fa.phase = phase;
     fa.loss_weight = p->loss_weight;
     fa.probe = probe;
     fa.probe_f = at<float2>(ws, q.o_probe_f);

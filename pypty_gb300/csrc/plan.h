@@ -20,7 +20,7 @@ struct Plan {
   int W, Ny, Nx, Z, Mo, Mp, N, nseq, Bb, nbatch, zm, ntx, nty, ntiles, nchunk, chunk;
   size_t o_tw, o_mask, o_mask_sc, o_prop, o_prop_edge, o_pyx, o_sx, o_sy, o_probe_f;
   size_t o_pos, o_corr, o_seq, o_obj, o_grad, o_obl, o_stack, o_gsum, o_fprobe, o_partial;
-  size_t o_lists, o_counts, o_loss_part, o_pos_part, o_sim, o_err, o_gbuf, o_psi, o_dldi, o_pgr, o_seg, o_gpark;
+  size_t o_lists, o_counts, o_loss_part, o_pos_part, o_sim, o_err, o_psi, o_dldi, o_pgr, o_seg, o_gpark;
   size_t total;
   int ckpt;   // kept slices every ckpt (256 windows)
   bool split;   // one batch with every position: pty_forward / pty_backward
@@ -30,7 +30,8 @@ struct Plan {
   // ib + 1's windows and scatters batch ib's gradients meanwhile; s_* are the buffer strides
   // in bytes
   int nbuf;
-  size_t s_obl, s_gsum, s_fprobe, s_stack;
+  size_t s_obl, s_gsum, s_fprobe, s_stack, s_psi, s_dldi;
+  bool halves;   // the whole pass runs as forward half, loss, adjoint half
   int per_step;   // one propagator table per slice step (slice_distances given, Z > 1)
   size_t o_steps;
   // scatter runs per tile (scatter_tiles_kernel groups): > 1 when tiles x slices give too few
@@ -40,8 +41,14 @@ struct Plan {
   size_t o_done;   // per (slice, tile) count of finished run blocks (sgroups > 1)
 };
 
-// blocks the scatter aims for: two per SM of a 152-SM GB300
-constexpr int kScatterBlocks = 304;
+// SMs of a GB300
+constexpr int kSMs = 152;
+
+// blocks the scatter aims for: two per SM
+constexpr int kScatterBlocks = 2 * kSMs;
+
+// blocks of the fused kernel that the GPU holds at once (64-px windows: two per SM)
+constexpr int resident_blocks(int W) { return W == 64 ? 2 * kSMs : kSMs; }
 
 // twiddle tables in global memory: W = 256 windows use the 128 tables of their sub-transforms
 inline int tw_count(int W) { return W == 64 ? Geo<64>::TW1 + Geo<64>::TW2 : Geo<128>::TW1 + Geo<128>::TW2; }
@@ -124,9 +131,19 @@ inline Plan make_plan(const pty_problem_t* p, bool split = false) {
   q.o_sim = take((size_t)q.Bb * WW * f4);
   q.o_err = take(sizeof(int));
   const bool w256 = q.W == 256;
-  q.o_gbuf = take(split && !w256 ? (size_t)q.Bb * q.Mp * q.Mo * WW * c8 : 0);
-  q.o_psi = take(w256 ? (size_t)q.Bb * q.Mp * q.Mo * WW * c8 : 0);
-  q.o_dldi = take(w256 ? (size_t)q.Bb * WW * f4 : 0);
+  // The whole pass of 64- and 128-px windows runs as its halves (see FusedPart) when a batch has
+  // several modes and about fills the GPU. The halves use the SMs that clusters leave idle and
+  // form the loss once per position, for two more launches (~10 us of a call). Whole pass against
+  // halves: 128 px, 768 blocks x 20 slices, four batches, 18.4 -> 16.4 ms; 128 blocks x 7 slices,
+  // three batches, 1036 -> 1004 us; 108 blocks x 3 slices 248 -> 251 us; 64 px, 768 blocks x 6
+  // slices 563 -> 522 us; 256 blocks x 8 slices 277 -> 286 us.
+  const int blocks = q.Bb * q.Mp;
+  q.halves = !w256 && !split && q.Mo == 1 && q.Mp > 1 && blocks > (q.W == 64 ? resident_blocks(64) : kSMs * 3 / 4);
+  const bool far = w256 || split || q.halves;
+  q.s_psi = align_up(far ? (size_t)q.Bb * q.Mp * q.Mo * WW * c8 : 0);
+  q.s_dldi = align_up(far ? (size_t)q.Bb * WW * f4 : 0);
+  q.o_psi = take(q.nbuf * q.s_psi);
+  q.o_dldi = take(q.nbuf * q.s_dldi);
   q.o_pgr = take(w256 && q.Mo > 1 ? (size_t)q.Bb * q.Mp * WW * c8 : 0);
   q.o_seg = take(q.ckpt > 1 ? (size_t)q.Bb * q.ckpt * WW * c8 : 0);
   q.o_gpark = take(q.ckpt > 1 ? (size_t)q.Bb * WW * c8 : 0);

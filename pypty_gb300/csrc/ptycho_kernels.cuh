@@ -315,11 +315,8 @@ __global__ void __launch_bounds__(Geo<W>::T) object_windows_kernel(WindowArgs a)
 // ------------------------------------------------------------------ fused multislice
 struct FusedArgs {
   int Z, Mp, Mo, algorithm, step_obj, step_probe, step_pos, probe_shift, simulate, use_edge;
-  int phase;                // 0: whole pass; 1: forward half; 2: adjoint half;
-                            // 3: forward multislice only (exit wave out); 4: adjoint from a given
-                            //    exit-wave gradient with a real-space probe gradient out
-  const float2* probe_b;    // per-position incoming probes, native real [Bb*Mp] (phase 3)
-  float2* exit_out;         // exit waves, native real [Bb*Mp*Mo] (phase 3)
+  const float2* probe_b;    // forward half: given incoming probes, native real [Bb*Mp]; or nullptr
+  float2* exit_out;         // forward half: exit waves out instead of the far field, native real [Bb*Mp*Mo]
   float loss_weight;
   const float2* probe;      // (W, W, Mp) reference layout (used without probe shift)
   const float2* probe_f;    // native frequency layout [Mp]
@@ -342,9 +339,10 @@ struct FusedArgs {
   float2* stack;            // input waves (256 windows: their conjugates), native real [Bb*Z*Mp*Mo]
   float2* gsum;             // object-gradient contributions, native real [Bb*Z*Mo*Mp] (probe mode innermost)
   float2* fprobe;           // FFT of the per-position probe gradient, native freq [Bb*Mp]
-  float2* gbuf;             // dL/d(exit wave) between the two halves, native real [Bb*Mp*Mo]
-  float2* psi;              // 256 windows: far-field wave per mode [Bb*Mp*Mo]
-  float* dldi;              // 256 windows: dL/dI between the two halves [Bb]
+  const float2* gbuf;       // adjoint half: a given dL/d(exit wave), native real [Bb*Mp*Mo], and a
+                            // real-space probe gradient out; or nullptr
+  float2* psi;              // halves: far-field wave per mode, native freq [Bb*Mp*Mo]
+  float* dldi;              // halves: dL/dI, native freq order of the packs [Bb]
   float2* pgr;              // 256 windows: object-mode sum of the probe gradient [Bb*Mp]
   int ckpt;                 // 256 windows: keep every ckpt-th slice's wave, recompute the rest
   float2* seg;              // 256 windows: recomputed waves of one segment [Bb*ckpt]
@@ -496,8 +494,15 @@ struct FusedSmem {
 // transform. The adjoint's O_z lands in the warp's part of the exchange buffer while the
 // inverse transform finishes its last register-only round; the adjoint's first step finds
 // psi_{Z-1} still in the side buffer.
-// PH = 0: the whole pass (phase 0) with every phase branch compiled out; PH = 1: a.phase at
-// run time (the split halves and the multislice_core phases).
+// PH_WHOLE: the whole pass. PH_FWD: steps 0..Z up to the far field, which goes to psi
+// (far_field_loss_kernel forms dL/dI from the modes' psi), or, with exit_out, up to the exit
+// wave (multislice_core.multislice). PH_ADJ: from psi and dL/dI, or from a given dL/d(exit wave)
+// (gbuf, multislice_core.multislice_grads), to the gradients. The halves need no cluster (with
+// one object mode): blocks of a position are independent, so they fill every SM, where clusters
+// of three leave one SM in eleven idle, and the loss is formed once per position instead of once
+// per mode.
+enum FusedPart : int { PH_WHOLE = 0, PH_FWD = 1, PH_ADJ = 2 };
+
 template <int W, int PH>
 __global__ void __launch_bounds__(Geo<W>::T, Geo<W>::MINB) fused_multislice_kernel(FusedArgs a) {
   using G = Geo<W>;
@@ -527,14 +532,13 @@ __global__ void __launch_bounds__(Geo<W>::T, Geo<W>::MINB) fused_multislice_kern
   cg::cluster_group cluster = cg::this_cluster();
   const int t = threadIdx.x;
   const int nmodes = a.Mp * a.Mo;
-  const int crank = (int)cluster.block_rank();
+  const int crank = PH == PH_WHOLE ? (int)cluster.block_rank() : (int)(blockIdx.x % nmodes);
   const int p = crank % a.Mp, m = crank / a.Mp;
   const int b = blockIdx.x / nmodes;
   const int gi = a.seq[b];
   const float dy = a.corr[2 * gi], dx = a.corr[2 * gi + 1];
   const int Z = a.Z;
   const bool adj_stack = a.step_obj && !a.simulate;   // the adjoint reads psi_z
-  const int phase = PH == 0 ? 0 : a.phase;
   const int warp = t >> 5, lane = t & 31;
   uint64_t *bar_x = bars + warp, *bar_side = bars + NW + warp;
   float4* wx = reinterpret_cast<float4*>(xbuf + warp * F::WPART);         // this warp's share of xbuf
@@ -563,7 +567,7 @@ __global__ void __launch_bounds__(Geo<W>::T, Geo<W>::MINB) fused_multislice_kern
   float2* sramp = reinterpret_cast<float2*>(smem + S::ramp_off);  // W = 64 only
   if constexpr (kLean) {
     // only passes that reach the far field (which waits for these copies) issue them
-    if (!a.simulate && a.measured && (phase <= 1)) {
+    if (PH == PH_WHOLE && !a.simulate && a.measured) {
       const float* src = a.measured + (size_t)gi * WW;
       if ((reinterpret_cast<uintptr_t>(src) & 15u) == 0) {
         for (int e = 4 * t; e < (int)WW; e += 4 * T) cp_async16(smeas + e, src + e);
@@ -631,25 +635,26 @@ __global__ void __launch_bounds__(Geo<W>::T, Geo<W>::MINB) fused_multislice_kern
   Win v;
   int side_next = -1;        // the slice whose window prefix the side buffer takes next
   bool side_held = false;    // the side buffer holds the next step's operand, waited for
-  float2* gb = a.gbuf + (((size_t)b * a.Mp + p) * a.Mo + m) * WW;
-  const bool adjoint_only = (phase == 2 || phase == 4);
-  const int s_begin = adjoint_only ? Z + 1 : 0;
-  const int s_end = (a.simulate || phase == 1 || phase == 3) ? Z + 1 : 2 * Z + 1;
-  if (adjoint_only) {
-    // adjoint half: resume from dL/d(exit wave) kept by the forward half
-    ld_native(gb, v);
-    issue_x(Z + 1);
+  const int s_begin = PH == PH_ADJ ? (a.gbuf ? Z + 1 : Z) : 0;
+  const int s_end = (a.simulate || PH == PH_FWD) ? Z + 1 : 2 * Z + 1;
+  if (PH == PH_ADJ) {
+    if (a.gbuf) {
+      ld_native(a.gbuf + (((size_t)b * a.Mp + p) * a.Mo + m) * WW, v);
+      issue_x(Z + 1);
+    }
     if (adj_stack) issue_side(stack_ptr(Z - 1));
   } else {
     issue_side(obl_ptr(0));
   }
   for (int s = s_begin; s < s_end; ++s) {
-    const bool fwd = (s >= 1 && s <= Z);
+    const bool fwd = PH == PH_ADJ ? false : PH == PH_FWD ? s >= 1 : (s >= 1 && s <= Z);
+    const bool far_start = PH == PH_ADJ && s == Z;   // resumes at the far field
     const int z = fwd ? s - 1 : 2 * Z - s;
 
     // ------------------------------------------------ real-space op
-    if (s == 0) {
-      if (PH != 0 && a.probe_b) {
+    if (far_start) {
+    } else if (PH != PH_ADJ && s == 0) {
+      if (PH == PH_FWD && a.probe_b) {
         ld_native(a.probe_b + ((size_t)b * a.Mp + p) * WW, v);
       } else if (!a.probe_shift) {
 #pragma unroll
@@ -680,14 +685,14 @@ __global__ void __launch_bounds__(Geo<W>::T, Geo<W>::MINB) fused_multislice_kern
         pcmul(v.re[j], v.im[j], make_float2(q.x, q.y), oi, pneg(oi));
       }
       // the adjoint's first step (the same slice) reads psi_z from the side buffer itself
-      if (adj_stack && !(z == Z - 1 && phase == 0)) store_side(stack_ptr(z));
+      if (adj_stack && !(z == Z - 1 && PH == PH_WHOLE)) store_side(stack_ptr(z));
       if (z + 1 < Z) side_next = z + 1;
       else side_held = true;
-      if (phase == 3 && z == Z - 1) {
+      if (PH == PH_FWD && a.exit_out && z == Z - 1) {
         st_native(a.exit_out + (((size_t)b * a.Mp + p) * a.Mo + m) * WW, v);   // the exit wave
         break;
       }
-    } else {
+    } else if (PH != PH_FWD) {
       if (adj_stack) {
         // psi_z: elements NST.. straight from global memory (this thread stored them in
         // the forward), the rest in the side buffer
@@ -731,7 +736,8 @@ __global__ void __launch_bounds__(Geo<W>::T, Geo<W>::MINB) fused_multislice_kern
       if (z == 0) {
         if (!(a.step_probe || a.step_pos)) break;
         if (a.Mo > 1) {
-          // probe gradient: sum over object modes (multislice_core.py:193-197)
+          // probe gradient: sum over object modes (multislice_core.py:193-197); with Mo > 1 the
+          // adjoint half runs in clusters too
           __syncthreads();
 #pragma unroll
           for (int i = 0; i < 32; ++i) xbuf[i * T + t] = wget(v, i);
@@ -748,7 +754,7 @@ __global__ void __launch_bounds__(Geo<W>::T, Geo<W>::MINB) fused_multislice_kern
           cluster.sync();
           if (m != 0) break;
         }
-        if (phase == 4) {   // interm_probe_grad of multislice_core.py:193-197, real space
+        if (PH == PH_ADJ && a.gbuf) {   // interm_probe_grad of multislice_core.py:193-197, real space
           if (a.step_probe) st_native(a.fprobe + ((size_t)b * a.Mp + p) * WW, v);
           break;
         }
@@ -756,7 +762,7 @@ __global__ void __launch_bounds__(Geo<W>::T, Geo<W>::MINB) fused_multislice_kern
     }
 
     // ------------------------------------------------ forward FFT
-    if (s > 0) {
+    if (s > 0 && !far_start) {
       __syncwarp();   // the warp has read its operands from the exchange and side buffers
       F::forward(v, xbuf, tw1, tw2);
       if (side_next >= 0) {   // refill the side buffer once its bulk store has read it
@@ -767,16 +773,27 @@ __global__ void __launch_bounds__(Geo<W>::T, Geo<W>::MINB) fused_multislice_kern
     }
 
     // ------------------------------------------------ frequency op
-    if (s == 0) {
+    if (far_start) {
+      // dL/dPsi = dL/dI * Psi * w (objective.py:595-597), both left by the forward half
+      ld_native(a.psi + (((size_t)b * a.Mp + p) * a.Mo + m) * WW, v);
+      const float2* di = reinterpret_cast<const float2*>(a.dldi + (size_t)b * WW) + wo;
+      const float2 lw = pdup(a.loss_weight);
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        const float2 d = di[j * 32];
+        v.re[j] = pmul(pmul(v.re[j], d), lw);
+        v.im[j] = pmul(pmul(v.im[j], d), lw);
+      }
+    } else if (PH != PH_ADJ && s == 0) {
       if (!a.probe_shift) continue;   // the unshifted probe is already in real space
       const float2* pf = a.probe_f + (size_t)p * WW;
       const float inv = 1.0f / (float)WW;
-      if (kLean && a.mask_bin) {
+      if (a.mask_bin) {
         const uint32_t mbits = sbits[t];
         visit_sep_ramp<W>(a, t, dy, dx, [&](auto I, int, int, float2 ramp) {
           constexpr int i = decltype(I)::value;
+          if constexpr (PH == PH_WHOLE && kLean) sramp[i * T + t] = ramp;   // serves the probe-gradient step too
           wset(v, i, ((mbits >> i) & 1u) ? cscale(cmul(native_at(pf, i, t), ramp), inv) : make_float2(0.f, 0.f));
-          sramp[i * T + t] = ramp;   // the same ramp serves the probe-gradient step (phase 0)
         });
       } else {
 #pragma unroll
@@ -785,7 +802,7 @@ __global__ void __launch_bounds__(Geo<W>::T, Geo<W>::MINB) fused_multislice_kern
           wset(v, i, cscale(cmul(native_at(pf, i, t), shift_ramp<W>(a, ky, kx, a.mask[ky * W + kx], dy, dx)), inv));
         }
       }
-    } else if (fwd && z < Z - 1) {
+    } else if (PH != PH_ADJ && fwd && z < Z - 1) {
       if (a.use_sep && !(z == 0 && a.use_edge)) {
         propagate_sep(v, false);
       } else {
@@ -793,7 +810,22 @@ __global__ void __launch_bounds__(Geo<W>::T, Geo<W>::MINB) fused_multislice_kern
                                         : ((z == 0 && a.use_edge) ? a.prop_edge : a.prop);
         mul_table<W>(v, pr, false);
       }
-    } else if (fwd) {
+    } else if (PH == PH_FWD && fwd) {
+      // far field: Psi = FFT(exit) * mask (objective.py:501-503); far_field_loss_kernel goes on
+      if (a.mask_bin) {
+        const uint32_t mbits = sbits[t];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+          const bool in0 = (mbits >> (2 * j)) & 1u, in1 = (mbits >> (2 * j + 1)) & 1u;
+          v.re[j] = make_float2(in0 ? v.re[j].x : 0.f, in1 ? v.re[j].y : 0.f);
+          v.im[j] = make_float2(in0 ? v.im[j].x : 0.f, in1 ? v.im[j].y : 0.f);
+        }
+      } else {
+        mul_real_table<W>(v, a.mask);
+      }
+      st_native(a.psi + (((size_t)b * a.Mp + p) * a.Mo + m) * WW, v);
+      break;
+    } else if (PH == PH_WHOLE && fwd) {
       // far field: Psi = FFT(exit) * mask, I = mean over modes |Psi|^2 (objective.py:501-512)
       if constexpr (kLean) cp_async_wait_all();   // the measured pattern; the cluster barrier below
                                                   // makes every thread's part visible
@@ -892,7 +924,7 @@ __global__ void __launch_bounds__(Geo<W>::T, Geo<W>::MINB) fused_multislice_kern
         v.im[j] = pmul(pmul(v.im[j], d), lw);
       }
       __syncthreads();   // the inverse transform's stores replace other threads' dL/dI
-    } else if (z > 0) {
+    } else if (PH != PH_FWD && z > 0) {
       if (a.use_sep && !(z == 1 && a.use_edge)) {
         propagate_sep(v, true);
       } else {
@@ -900,39 +932,47 @@ __global__ void __launch_bounds__(Geo<W>::T, Geo<W>::MINB) fused_multislice_kern
                                         : ((z == 1 && a.use_edge) ? a.prop_edge : a.prop);
         mul_table<W>(v, pr, true);
       }
-    } else {
+    } else if (PH != PH_FWD) {
       // probe-gradient spectrum with the shift adjoint, position gradient (objective.py:641-656)
       const float2* pf = a.probe_f + (size_t)p * WW;
       FSum gy_c, gx_c;
-      if (kLean && a.probe_shift && a.mask_bin && phase == 0) {
-        // the first step's ramp, kept in shared memory by this thread
+      // this element's spectrum times the conjugate ramp, and its share of the position gradient:
+      // Re(smyx * conj(Pf) * F) with smyx = i*s*mask  ->  -(s*mask) * Im(conj(Pf) * F)
+      auto probe_element = [&](auto I, int ky, int kx, float2 ramp, float mk) {
+        constexpr int i = decltype(I)::value;
+        const float2 g = cmulc(wget(v, i), cscale(ramp, mk));
+        wset(v, i, g);
+        if (a.step_pos) {
+          const float im = cmulc(g, native_at(pf, i, t)).y;
+          gy_c += -(a.sy[ky] * mk) * im;
+          gx_c += -(a.sx[kx] * mk) * im;
+        }
+      };
+      if (a.probe_shift && a.mask_bin) {
         const uint32_t mbits = sbits[t];
-#pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          const int ky = G::fky(t, i), kx = G::fkx(t, i);
-          const float mk = ((mbits >> i) & 1u) ? 1.0f : 0.0f;
-          const float2 g = cmulc(wget(v, i), cscale(sramp[i * T + t], mk));
-          wset(v, i, g);
-          if (a.step_pos) {   // as below
-            const float im = cmulc(g, native_at(pf, i, t)).y;
-            gy_c += -(a.sy[ky] * mk) * im;
-            gx_c += -(a.sx[kx] * mk) * im;
-          }
+        if constexpr (PH == PH_WHOLE && kLean) {   // the first step's ramp, kept in shared memory
+          static_for<0, 32>([&](auto I) {
+            constexpr int i = decltype(I)::value;
+            probe_element(I, G::fky(t, i), G::fkx(t, i), sramp[i * T + t], ((mbits >> i) & 1u) ? 1.0f : 0.0f);
+          });
+        } else {
+          visit_sep_ramp<W>(a, t, dy, dx, [&](auto I, int ky, int kx, float2 ramp) {
+            probe_element(I, ky, kx, ramp, ((mbits >> decltype(I)::value) & 1u) ? 1.0f : 0.0f);
+          });
         }
       } else if (a.probe_shift) {
-#pragma unroll
-        for (int i = 0; i < 32; ++i) {
+        static_for<0, 32>([&](auto I) {
+          constexpr int i = decltype(I)::value;
           const int ky = G::fky(t, i), kx = G::fkx(t, i);
           const float mk = a.mask[ky * W + kx];
           const float2 g = cmulc(wget(v, i), shift_ramp<W>(a, ky, kx, mk, dy, dx));
           wset(v, i, g);
           if (a.step_pos) {
-            // Re(smyx * conj(Pf) * F) with smyx = i*s*mask  ->  -(s*mask) * Im(conj(Pf) * F)
             const float im = cmulc(g, native_at(pf, i, t)).y;
             gy_c += -(a.sy[ky] * mk) * im;
             gx_c += -(a.sx[kx] * mk) * im;
           }
-        }
+        });
       }
       if (a.step_probe) st_native(a.fprobe + ((size_t)b * a.Mp + p) * WW, v);
       if (a.step_pos) {
@@ -953,7 +993,7 @@ __global__ void __launch_bounds__(Geo<W>::T, Geo<W>::MINB) fused_multislice_kern
       if (s + 1 > Z) {     // the adjoint steps read O_z from the exchange buffer
         __syncwarp();      // the warp has finished reading its part
         // the adjoint's side-buffer copies read the stack's bulk-stored parts back
-        if (s == Z && lane == 0) bulk_wait_all();
+        if (PH == PH_WHOLE && s == Z && lane == 0) bulk_wait_all();
         issue_x(s + 1);
       }
       // every block asks for its operands at about the same time: bring what the next steps
@@ -977,7 +1017,57 @@ __global__ void __launch_bounds__(Geo<W>::T, Geo<W>::MINB) fused_multislice_kern
     F::inverse_tail(v);
   }
   if (lane == 0) bulk_wait_all();   // the bulk stores are complete before the block exits
-  if (phase == 1) st_native(gb, v);   // forward half: keep dL/d(exit wave)
+}
+
+// ------------------------------------------------------------------ loss of the halves
+// Mean-over-modes intensity, loss and dL/dI (objective.py:509-587) of one position per block from
+// the far-field waves that PH_FWD left in psi; dL/dI goes to dldi in the packs' native order, or
+// with simulate the pattern to sim_out. The modes' sum, the pixels' order over threads and the
+// block sums are those of the whole-pass kernel, so both give the same bits.
+template <int W>
+__global__ void __launch_bounds__(Geo<W>::T) far_field_loss_kernel(FusedArgs a) {
+  using G = Geo<W>;
+  constexpr size_t WW = (size_t)W * W;
+  __shared__ double red[64];
+  const int t = threadIdx.x, b = blockIdx.x, nmodes = a.Mp * a.Mo;
+  const float inv_modes = 1.0f / (float)nmodes;
+  const float* meas = a.simulate ? nullptr : a.measured + (size_t)a.seq[b] * WW;
+  float2* dldi = reinterpret_cast<float2*>(a.dldi + (size_t)b * WW) + nword(0, t);
+  FSum lsum_c, ssum_c;
+#pragma unroll 4
+  for (int j = 0; j < 16; ++j) {
+    const int d0 = detector_index<W>(t, 2 * j), d1 = detector_index<W>(t, 2 * j + 1);
+    float2 mv = make_float2(0.f, 0.f);
+    if (!a.simulate) mv = make_float2(meas[d0], meas[d1]);
+    float2 acc = make_float2(0.f, 0.f);
+    for (int r = 0; r < nmodes; ++r) {   // m ascending, p innermost, as the cluster's ranks
+      const int p = r % a.Mp, m = r / a.Mp;
+      const float4 q = reinterpret_cast<const float4*>(a.psi + (((size_t)b * a.Mp + p) * a.Mo + m) * WW)[nword(j, t)];
+      const float2 re = make_float2(q.x, q.y), im = make_float2(q.z, q.w);
+      acc = padd(acc, pfma(im, im, pmul(re, re)));
+    }
+    const float I0 = (nmodes == 1) ? acc.x : acc.x * inv_modes, I1 = (nmodes == 1) ? acc.y : acc.y * inv_modes;
+    if (a.simulate) {
+      a.sim_out[(size_t)b * WW + d0] = I0;
+      a.sim_out[(size_t)b * WW + d1] = I1;
+      continue;
+    }
+    float2 d;
+    d.x = loss_pixel(a.algorithm, I0, mv.x, lsum_c, ssum_c);
+    d.y = loss_pixel(a.algorithm, I1, mv.y, lsum_c, ssum_c);
+    if (nmodes > 1) {                                // objective.py:586-587
+      d.x = d.x / (float)nmodes;
+      d.y = d.y / (float)nmodes;
+    }
+    dldi[j * 32] = d;
+  }
+  if (a.simulate) return;
+  double lsum = lsum_c.value(), ssum = ssum_c.value();
+  block_sum2(lsum, ssum, red);
+  if (t == 0) {
+    a.loss_part[2 * b] = lsum;
+    a.loss_part[2 * b + 1] = ssum;
+  }
 }
 
 // ------------------------------------------------------------------ reference-layout windows
