@@ -9,183 +9,22 @@
 // loss) go through fixed per-block partial sums and a fixed-order final sum: training is
 // deterministic run to run.
 //
-// conv3x3_kernel: a CTA computes a 32 x 32 pixel tile for 16 output channels; each thread a
-// 2 x 2 pixel quad for those 16 channels (64 FP32 accumulators); input channels stream through
-// shared memory 8 at a time with a one-pixel zero-padded halo; the weights of a chunk are read
-// as float4 broadcasts (16 FMAs per weight load). The transposed-and-flipped weight view gives
-// the data gradient with the same kernel.
+// The 3x3 convolutions, their data and weight gradients run on the tensor cores (conv_mma.cuh).
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
 #include <cstdint>
 
+#include "conv_mma.cuh"
 #include "plan.h"
 
 namespace pty {
 namespace nn {
 
-typedef __nv_bfloat16 bf16;
-
 __device__ __forceinline__ float ld(const bf16* p) { return __bfloat162float(*p); }
 __device__ __forceinline__ bf16 to_bf(float x) { return __float2bfloat16_rn(x); }
 
-constexpr int TS = 32;    // output tile edge
-constexpr int COT = 16;   // output channels per CTA
-constexpr int CIT = 8;    // input channels per shared-memory chunk
-constexpr int HALO = TS + 2;
-
-// TRANS = 0: out[n][o] = act(b[o] + sum_i sum_t w[o][i][t] x[n][i][p + off(t)])   (forward)
-// TRANS = 1: out[n][o] =          sum_i sum_t w[i][o][8 - t] x[n][i][p + off(t)]    (data gradient;
-//            o runs over the layer's input channels, i over its output channels)
-template <int TRANS, int RELU>
-__global__ void __launch_bounds__(256) conv3x3_kernel(const bf16* __restrict__ x, const float* __restrict__ w,
-                                                      const float* __restrict__ bias, bf16* __restrict__ out, int Ci,
-                                                      int Co, int H, int Wd) {
-  __shared__ float xs[CIT][HALO][HALO + 1];
-  __shared__ __align__(16) float ws[CIT][9][COT];
-  const int tiles_x = Wd / TS;
-  const int ty0 = (blockIdx.x / tiles_x) * TS, tx0 = (blockIdx.x % tiles_x) * TS;
-  const int o0 = blockIdx.y * COT, n = blockIdx.z;
-  const int t = threadIdx.x, qx = (t & 15) * 2, qy = (t >> 4) * 2;
-  float acc[4][COT];
-#pragma unroll
-  for (int p = 0; p < 4; ++p)
-#pragma unroll
-    for (int c = 0; c < COT; ++c) acc[p][c] = 0.f;
-  const size_t plane = (size_t)H * Wd;
-  for (int i0 = 0; i0 < Ci; i0 += CIT) {
-    __syncthreads();
-    for (int e = t; e < CIT * HALO * HALO; e += 256) {
-      const int ci = e / (HALO * HALO), r = (e / HALO) % HALO, c = e % HALO;
-      const int y = ty0 + r - 1, xx = tx0 + c - 1;
-      float v = 0.f;
-      if (i0 + ci < Ci && y >= 0 && y < H && xx >= 0 && xx < Wd) v = ld(x + ((size_t)n * Ci + i0 + ci) * plane + (size_t)y * Wd + xx);
-      xs[ci][r][c] = v;
-    }
-    for (int e = t; e < CIT * 9 * COT; e += 256) {
-      const int ci = e / (9 * COT), tap = (e / COT) % 9, co = e % COT;
-      const int i = i0 + ci, o = o0 + co;
-      float v = 0.f;
-      if (i < Ci && o < Co) v = TRANS ? w[((size_t)i * Co + o) * 9 + (8 - tap)] : w[((size_t)o * Ci + i) * 9 + tap];
-      ws[ci][tap][co] = v;
-    }
-    __syncthreads();
-#pragma unroll 2
-    for (int ci = 0; ci < CIT; ++ci) {
-#pragma unroll
-      for (int tap = 0; tap < 9; ++tap) {
-        const int dy = tap / 3, dx = tap % 3;
-        const float v0 = xs[ci][qy + dy][qx + dx], v1 = xs[ci][qy + dy][qx + 1 + dx];
-        const float v2 = xs[ci][qy + 1 + dy][qx + dx], v3 = xs[ci][qy + 1 + dy][qx + 1 + dx];
-        const float4* wp = reinterpret_cast<const float4*>(&ws[ci][tap][0]);
-#pragma unroll
-        for (int c4 = 0; c4 < COT / 4; ++c4) {
-          const float4 wv = wp[c4];
-          const float wl[4] = {wv.x, wv.y, wv.z, wv.w};
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            acc[0][4 * c4 + j] = fmaf(wl[j], v0, acc[0][4 * c4 + j]);
-            acc[1][4 * c4 + j] = fmaf(wl[j], v1, acc[1][4 * c4 + j]);
-            acc[2][4 * c4 + j] = fmaf(wl[j], v2, acc[2][4 * c4 + j]);
-            acc[3][4 * c4 + j] = fmaf(wl[j], v3, acc[3][4 * c4 + j]);
-          }
-        }
-      }
-    }
-  }
-#pragma unroll
-  for (int c = 0; c < COT; ++c) {
-    const int o = o0 + c;
-    if (o >= Co) break;
-    const float b = (!TRANS && bias) ? bias[o] : 0.f;
-    bf16* op = out + ((size_t)n * Co + o) * plane;
-#pragma unroll
-    for (int p = 0; p < 4; ++p) {
-      float v = acc[p][c] + b;
-      if (RELU) v = fmaxf(v, 0.f);
-      const int y = ty0 + qy + (p >> 1), xx = tx0 + qx + (p & 1);
-      op[(size_t)y * Wd + xx] = to_bf(v);
-    }
-  }
-}
-
-// Weight and bias gradients of a 3x3 convolution, per (32 x 32 tile, image) partial sums:
-//   part[blk][o][i][t] = sum_{p in tile} dy[n][o][p] x[n][i][p + off(t)],  pb[blk][o] = sum dy[n][o][p]
-// grid (tiles * N, Co / COT, Ci / CIT); thread = (o, i) pair of the CTA's 16 x 8 block, half the rows.
-struct WgradSmem {
-  float xs[CIT][HALO][HALO + 1];
-  float ds[COT][TS][TS + 1];
-  float red[256][10];
-};
-
-__global__ void __launch_bounds__(256) conv3x3_wgrad_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ x,
-                                                            float* __restrict__ part, float* __restrict__ pbias,
-                                                            int Ci, int Co, int H, int Wd, int N) {
-  extern __shared__ __align__(16) unsigned char wg_smem[];
-  WgradSmem& S = *reinterpret_cast<WgradSmem*>(wg_smem);
-  auto& xs = S.xs;
-  auto& ds = S.ds;
-  auto& red = S.red;
-  const int tiles_x = Wd / TS, tiles = (H / TS) * tiles_x;
-  const int tile = blockIdx.x % tiles, n = blockIdx.x / tiles;
-  const int ty0 = (tile / tiles_x) * TS, tx0 = (tile % tiles_x) * TS;
-  const int o0 = blockIdx.y * COT, i0 = blockIdx.z * CIT;
-  const int t = threadIdx.x;
-  const size_t plane = (size_t)H * Wd;
-  for (int e = t; e < CIT * HALO * HALO; e += 256) {
-    const int ci = e / (HALO * HALO), r = (e / HALO) % HALO, c = e % HALO;
-    const int y = ty0 + r - 1, xx = tx0 + c - 1;
-    float v = 0.f;
-    if (i0 + ci < Ci && y >= 0 && y < H && xx >= 0 && xx < Wd) v = ld(x + ((size_t)n * Ci + i0 + ci) * plane + (size_t)y * Wd + xx);
-    xs[ci][r][c] = v;
-  }
-  for (int e = t; e < COT * TS * TS; e += 256) {
-    const int co = e / (TS * TS), r = (e / TS) % TS, c = e % TS;
-    float v = 0.f;
-    if (o0 + co < Co) v = ld(dy + ((size_t)n * Co + o0 + co) * plane + (size_t)(ty0 + r) * Wd + tx0 + c);
-    ds[co][r][c] = v;
-  }
-  __syncthreads();
-  const int pair = t & 127, half = t >> 7;
-  const int co = pair >> 3, ci = pair & 7;
-  float a[9], sb = 0.f;
-#pragma unroll
-  for (int k = 0; k < 9; ++k) a[k] = 0.f;
-  for (int r = half * 16; r < half * 16 + 16; ++r) {
-    // sliding 3x3 window of x around (r, c): columns c-1, c, c+1 of rows r-1, r, r+1 (halo offset +1)
-    float w0[3] = {xs[ci][r][0], xs[ci][r + 1][0], xs[ci][r + 2][0]};
-    float w1[3] = {xs[ci][r][1], xs[ci][r + 1][1], xs[ci][r + 2][1]};
-    for (int c = 0; c < TS; ++c) {
-      const float w2[3] = {xs[ci][r][c + 2], xs[ci][r + 1][c + 2], xs[ci][r + 2][c + 2]};
-      const float d = ds[co][r][c];
-      sb += d;
-#pragma unroll
-      for (int dyy = 0; dyy < 3; ++dyy) {
-        a[dyy * 3 + 0] = fmaf(d, w0[dyy], a[dyy * 3 + 0]);
-        a[dyy * 3 + 1] = fmaf(d, w1[dyy], a[dyy * 3 + 1]);
-        a[dyy * 3 + 2] = fmaf(d, w2[dyy], a[dyy * 3 + 2]);
-      }
-#pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        w0[k] = w1[k];
-        w1[k] = w2[k];
-      }
-    }
-  }
-#pragma unroll
-  for (int k = 0; k < 9; ++k) red[t][k] = a[k];
-  red[t][9] = sb;
-  __syncthreads();
-  if (half == 0) {
-    const int o = o0 + co, i = i0 + ci;
-    const size_t blk = blockIdx.x;
-    if (o < Co && i < Ci) {
-#pragma unroll
-      for (int k = 0; k < 9; ++k) part[((blk * Co + o) * Ci + i) * 9 + k] = red[t][k] + red[t + 128][k];
-    }
-    if (ci == 0 && blockIdx.z == 0 && o < Co) pbias[blk * Co + o] = red[t][9] + red[t + 128][9];
-  }
-}
+constexpr int TS = 32;    // image extents are multiples of this
 
 // dst[e] = sum_b src[b][e] in ascending b (the fixed-order reduction of per-block partials)
 __global__ void reduce_blocks_kernel(const float* __restrict__ src, float* __restrict__ dst, int nblk, long long n) {
@@ -463,13 +302,16 @@ int pty_nn_conv3x3(const void* x, const float* w, const float* bias, void* out, 
   if (!x || !w || !out || N <= 0 || Ci <= 0 || Co <= 0) return PTY_ERR_INVALID;
   if (H % TS || W % TS) return PTY_ERR_UNSUPPORTED;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const dim3 grid((H / TS) * (W / TS), (Co + COT - 1) / COT, N);
   const bf16* xb = static_cast<const bf16*>(x);
   bf16* ob = static_cast<bf16*>(out);
+  using C = ConvCfg;
+  const dim3 grid((H / C::T) * (W / C::T), (Co + C::CO - 1) / C::CO, N);
+  const int wide = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(out)) & 3) == 0;
+  const int wide4 = Ci % 4 == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0;   // four channels' taps as 16-byte words
+  auto kernel = transpose ? conv3x3_mma_kernel<1, 0> : relu ? conv3x3_mma_kernel<0, 1> : conv3x3_mma_kernel<0, 0>;
+  if (set_smem(kernel, C::SMEM)) return PTY_ERR_CUDA;
   prof_mark(st, KID_NN);
-  if (transpose) conv3x3_kernel<1, 0><<<grid, 256, 0, st>>>(xb, w, nullptr, ob, Ci, Co, H, W);
-  else if (relu) conv3x3_kernel<0, 1><<<grid, 256, 0, st>>>(xb, w, bias, ob, Ci, Co, H, W);
-  else conv3x3_kernel<0, 0><<<grid, 256, 0, st>>>(xb, w, bias, ob, Ci, Co, H, W);
+  kernel<<<grid, C::THREADS, C::SMEM, st>>>(xb, w, transpose ? nullptr : bias, ob, Ci, Co, H, W, wide, wide4);
   prof_mark(st, -1);
   return launch_ok();
 }
@@ -486,20 +328,19 @@ int pty_nn_conv3x3_wgrad(const void* dy, const void* x, float* dw, float* db, in
   if (!dy || !x || !dw || !db || !workspace) return PTY_ERR_INVALID;
   if (H % TS || W % TS) return PTY_ERR_UNSUPPORTED;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const int blocks = N * (H / TS) * (W / TS);
+  using C = WgradCfg;
+  const int ct = (Co + C::CO - 1) / C::CO, it = (Ci + C::CI - 1) / C::CI;
+  // pixel shares: two CTAs per SM in all, and no more partial sums than the workspace holds
+  const int blocks = std::max(1, std::min(N * (H / TS) * (W / TS), 2 * kSMs / (ct * it)));
   float* part = workspace;
   float* pb = workspace + (size_t)blocks * Co * Ci * 9;
-  if (cudaFuncSetAttribute(conv3x3_wgrad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(WgradSmem)) !=
-      cudaSuccess)
-    return PTY_ERR_CUDA;
+  const int wide = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(dy)) & 3) == 0;
+  if (set_smem(conv3x3_wgrad_mma_kernel, C::SMEM)) return PTY_ERR_CUDA;
   prof_mark(st, KID_NN);
-  conv3x3_wgrad_kernel<<<dim3(blocks, (Co + COT - 1) / COT, (Ci + CIT - 1) / CIT), 256, sizeof(WgradSmem), st>>>(
-      static_cast<const bf16*>(dy), static_cast<const bf16*>(x), part, pb, Ci, Co, H, W, N);
-  const long long nw = (long long)Co * Ci * 9;
+  conv3x3_wgrad_mma_kernel<<<dim3(blocks, ct, it), C::THREADS, C::SMEM, st>>>(
+      static_cast<const bf16*>(dy), static_cast<const bf16*>(x), part, pb, Ci, Co, H, W, N, wide);
   prof_mark(st, KID_NN);
-  reduce_blocks_kernel<<<nblk(nw), 256, 0, st>>>(part, dw, blocks, nw);
-  prof_mark(st, KID_NN);
-  reduce_blocks_kernel<<<nblk(Co), 256, 0, st>>>(pb, db, blocks, Co);
+  wgrad_reduce_kernel<<<nblk((long long)Co * Ci * 9 + Co), 256, 0, st>>>(part, pb, dw, db, blocks, Ci, Co);
   prof_mark(st, -1);
   return launch_ok();
 }
