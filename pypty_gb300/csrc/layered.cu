@@ -809,12 +809,12 @@ __global__ void var_tilted_mul_kernel(float2* __restrict__ x, TiltArgs t, PropAr
 // per-position propagators (and their edge powers) of one batch, tabulated once and used by
 // every propagation step of the batch   grid (WW / EB, Bn)
 __global__ void var_pos_prop_table_kernel(TiltArgs t, PropArgs a, float2* __restrict__ tab,
-                                          float2* __restrict__ tab_edge) {
+                                          float2* __restrict__ tab_edge, float scale) {
   const int u = blockIdx.x * EB + threadIdx.x, b = blockIdx.y;
   const size_t WW = (size_t)a.W * a.W;
   const float* row = tilt_row(t, b);
-  tab[b * WW + u] = tilted_prop(a, row, u, false);
-  if (tab_edge) tab_edge[b * WW + u] = tilted_prop(a, row, u, true);
+  tab[b * WW + u] = cscale(tilted_prop(a, row, u, false), scale);
+  if (tab_edge) tab_edge[b * WW + u] = cscale(tilted_prop(a, row, u, true), scale);
 }
 
 // x[b][k] *= tab[b] (conj: conj(tab[b]))   grid (WW / EB, nper, Bn)
@@ -926,24 +926,71 @@ __global__ void __launch_bounds__(1024) var_tilt_adj_kernel(float2* __restrict__
 }
 
 // tilt gradient rows from the per-position partials, in sequence order
-// (objective.py:616-619, 635-639, 668-673; multislice_core.py:181-182)   one block
-__global__ void var_tilt_finalize_kernel(const double* __restrict__ part, const int* __restrict__ seq, int nseq,
-                                         int n_rows, int single, int use_before, int use_inside, int use_after,
-                                         float* __restrict__ grad) {
-  if (threadIdx.x != 0) return;
-  for (int i = 0; i < n_rows * 6; ++i) grad[i] = 0.0f;
-  for (int s = 0; s < nseq; ++s) {
-    float* g = grad + (single ? 0 : (size_t)seq[s] * 6);
-    const double* pp = part + (size_t)s * 6;
-    for (int c = 0; c < 6; ++c) {
-      const bool on = c < 2 ? use_before : (c < 4 ? use_inside : use_after);
-      if (!on) continue;
-      // before / after: one row sums the positions, per-position rows are assigned; inside
-      // terms accumulate
-      if (single || (c >= 2 && c < 4)) g[c] += (float)pp[c];
-      else g[c] = (float)pp[c];
+// (objective.py:616-619, 635-639, 668-673; multislice_core.py:181-182). Bound by the latency of
+// its loads: a thread per row (or per column of a single row) reads the sequence a block at a time;
+// one thread walking 144 rows in global memory took 83 us, this 18.   grid n_rows / 256 (single: 1)
+__global__ void __launch_bounds__(256) var_tilt_finalize_kernel(const double* __restrict__ part,
+                                                                const int* __restrict__ seq, int nseq, int n_rows,
+                                                                int single, int use_before, int use_inside,
+                                                                int use_after, float* __restrict__ grad) {
+  __shared__ int sseq[256];
+  auto on = [&](int c) { return c < 2 ? use_before : (c < 4 ? use_inside : use_after); };
+  if (single) {   // one row: a thread per column sums the positions in order
+    const int c = threadIdx.x;
+    if (blockIdx.x != 0 || c >= 6) return;
+    float g = 0.0f;
+    if (on(c)) {
+#pragma unroll 8
+      for (int s = 0; s < nseq; ++s) g += (float)part[(size_t)s * 6 + c];
+    }
+    grad[c] = g;
+    return;
+  }
+  // a thread per row: its entries of the sequence in order; before / after columns are assigned,
+  // inside columns accumulate
+  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+  float g[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  for (int s0 = 0; s0 < nseq; s0 += 256) {
+    __syncthreads();
+    if (s0 + (int)threadIdx.x < nseq) sseq[threadIdx.x] = seq[s0 + threadIdx.x];
+    __syncthreads();
+    const int n = min(256, nseq - s0);
+    for (int k = 0; k < n; ++k) {
+      if (sseq[k] != r) continue;
+      const double* pp = part + (size_t)(s0 + k) * 6;
+#pragma unroll
+      for (int c = 0; c < 6; ++c) {
+        if (!on(c)) continue;
+        g[c] = (c >= 2 && c < 4) ? g[c] + (float)pp[c] : (float)pp[c];
+      }
     }
   }
+  if (r < n_rows)
+#pragma unroll
+    for (int c = 0; c < 6; ++c) grad[(size_t)r * 6 + c] = g[c];
+}
+
+// host values into device memory without a pageable copy
+struct StepWeights {
+  static constexpr int N = 64;
+  float w[N];
+};
+__global__ void step_weights_kernel(StepWeights a, int n, float* __restrict__ out) {
+  if ((int)threadIdx.x < n) out[threadIdx.x] = a.w[threadIdx.x];
+}
+
+// the fused adjoint's inside-tilt sums of a batch, modes in order   grid Bn / 128, block 128
+__global__ void var_inside_sum_kernel(const double* __restrict__ tilt_part, int Bn, int nm, double sh,
+                                      double* __restrict__ part) {
+  const int b = blockIdx.x * blockDim.x + threadIdx.x;
+  if (b >= Bn) return;
+  double gy = 0.0, gx = 0.0;
+  for (int k = 0; k < nm; ++k) {
+    gy += tilt_part[2 * ((size_t)b * nm + k)];
+    gx += tilt_part[2 * ((size_t)b * nm + k) + 1];
+  }
+  part[(size_t)b * 6 + 2] += sh * gy;
+  part[(size_t)b * 6 + 3] += sh * gx;
 }
 
 // ------------------------------------------------------------------ plan
@@ -961,6 +1008,15 @@ struct LPlan {
   // beam tilts
   int n_rows, single_tilt, same_prop, before, after, inside_grad, step_tilts;
   int pos_prop;   // per-position propagator tables (per-position inside tilts that apply)
+  // the multislice part runs on the fused kernel's halves (var_forward, var_adjoint): 64- and 128-px
+  // windows, FP32 transforms, and not a propagator per position and step. A wave then stays in its
+  // block's registers from the first slice to the last, where a kernel per slice and step reads and
+  // writes every window: 128 px, 144 positions, 2 modes, 10 slices, a tilt per position 3.50 -> 1.79 ms;
+  // 64 px, 135 positions, 3 modes, 6 slices in near field 0.67 -> 0.53 ms. A propagator per position
+  // and step would be a table of Bb * (Z - 1) windows, and a window of 256 px takes a cluster.
+  int fused;
+  int sgroups;      // scatter runs per tile
+  size_t o_scpart, o_done, o_tilt_part, o_tilt_w, o_err;
   size_t o_tilts, o_tgrid, o_spec, o_fexit, o_exitb, o_pbt, o_pft, o_tpart, o_pprop, o_pprop_edge;
 };
 
@@ -1007,8 +1063,6 @@ inline LPlan make_lplan(const pty_problem_t* p, int engine, const pty_variant_t*
   q.o_grad = take((size_t)q.zm * q.Ny * q.Nx * c8);
   const size_t nobw = (size_t)q.Bb * q.zm, nwave = (size_t)q.Bb * q.Mp * q.Mo;
   q.o_ob = take(nobw * WWs * c8);
-  q.o_tmp = take(nobw * WWs * c8);
-  q.o_dob = take(nobw * WWs * c8);
   q.o_stack = take((size_t)q.Z * nwave * WWs * c8);
   q.o_psi = take(nwave * WWs * c8);
   q.o_psi2 = take(nwave * WWs * c8);
@@ -1064,7 +1118,20 @@ inline LPlan make_lplan(const pty_problem_t* p, int engine, const pty_variant_t*
     q.pos_prop = !q.same_prop || (q.per_step && !q.single_tilt);
     q.o_pprop = take(q.pos_prop ? (size_t)q.Bb * WWs * c8 : 0);
     q.o_pprop_edge = take(q.pos_prop && edge ? (size_t)q.Bb * WWs * c8 : 0);
+    q.fused = engine == PTY_DFT_FP32_FFT && q.W <= 128 && !(q.pos_prop && q.per_step);
   }
+  q.o_dob = take((q.fused ? q.Mp : 1) * nobw * WWs * c8);   // one contribution window per probe mode
+  q.o_tmp = take((q.fused ? 0 : nobw) * WWs * c8);
+  q.o_tilt_part = take(q.fused && q.inside_grad ? nwave * 2 * sizeof(double) : 0);
+  q.o_tilt_w = take(q.fused && q.inside_grad ? (size_t)q.Z * sizeof(float) : 0);
+  q.o_err = take(q.fused ? sizeof(int) : 0);
+  q.sgroups = 1;
+  if (q.fused) {
+    const int cells = q.ntiles * q.zm;
+    q.sgroups = std::max(1, std::min({(kScatterBlocks + cells - 1) / cells, std::max(1, q.Bb / 8), 32}));
+  }
+  q.o_scpart = take(q.sgroups > 1 ? (size_t)q.sgroups * q.ntiles * q.zm * kTileSize * kTileSize * c8 : 0);
+  q.o_done = take(q.sgroups > 1 ? (size_t)q.ntiles * q.zm * sizeof(int) : 0);
   size_t db = 0;
   const size_t maxwin = nobw > nwave ? nobw : nwave;
   const int32_t nmax = (int32_t)(maxwin > (size_t)q.Mp ? maxwin : (size_t)q.Mp);
@@ -1328,6 +1395,28 @@ struct Run {
     }
     // distance of slice step z (the step from slice z to z + 1)
     auto step_distance = [&](int z) { return q.per_step ? p->slice_distances[z] : p->slice_distance; };
+    // the inside-tilt gradient's factor of step z: -4 pi d / W^2 in float32, d (the step's distance)
+    // times the edge multiplier on the thick step (multislice_core.py:164-180)
+    auto tilt_sh = [&](int z) {
+      const float dist = z == 0 && ta.use_edge ? step_distance(z) * p->edge_mult : step_distance(z);
+      return fdiv_host((float)-12.566370614359172 * dist, (float)WW);
+    };
+    const float tilt_base = q.Z > 1 && tilt_sh(0) != 0.0f ? tilt_sh(0) : 1.0f;
+    if (q.fused) {
+      if (cudaMemsetAsync(at<int>(ws, q.o_err), 0, sizeof(int), st) != cudaSuccess) return PTY_ERR_CUDA;
+      if (q.sgroups > 1 &&
+          cudaMemsetAsync(at<int>(ws, q.o_done), 0, (size_t)q.ntiles * q.zm * sizeof(int), st) != cudaSuccess)
+        return PTY_ERR_CUDA;
+      if (q.inside_grad && q.Z > 1) {
+        // the steps' factors relative to step 0's (tilt_base)
+        StepWeights sw{};
+        for (int z0 = 0; z0 < q.Z - 1; z0 += StepWeights::N) {
+          const int n = std::min(StepWeights::N, q.Z - 1 - z0);
+          for (int k = 0; k < n; ++k) sw.w[k] = fdiv_host(tilt_sh(z0 + k), tilt_base);
+          step_weights_kernel<<<1, StepWeights::N, 0, st>>>(sw, n, at<float>(ws, q.o_tilt_w) + z0);
+        }
+      }
+    }
     float2* planes = at<float2>(ws, q.o_planes);
     float2* pf = at<float2>(ws, q.o_pf);
     prof_mark(st, KID_LAYOUT);
@@ -1385,9 +1474,11 @@ struct Run {
       const int Bn = q.nseq - i0 < q.Bb ? q.nseq - i0 : q.Bb;
       const int* seq_b = at<int>(ws, q.o_seq) + i0;
       // object windows, band-limited (objective.py:436-441)
-      prof_mark(st, KID_OBJECT_WINDOWS);
-      gather_kernel<<<grid(q.zm, Bn), EB, 0, st>>>(at<float2>(ws, q.o_obj), ob, d_pos, seq_b, W, q.Ny, q.Nx, q.zm);
-      if ((rc = band_limit(ob, tmp, (long long)Bn * q.zm))) return rc;
+      if (!q.fused) {
+        prof_mark(st, KID_OBJECT_WINDOWS);
+        gather_kernel<<<grid(q.zm, Bn), EB, 0, st>>>(at<float2>(ws, q.o_obj), ob, d_pos, seq_b, W, q.Ny, q.Nx, q.zm);
+        if ((rc = band_limit(ob, tmp, (long long)Bn * q.zm))) return rc;
+      }
       // incoming probe per position (objective.py:469-476)
       const float2* pin = planes;
       size_t pin_stride = 0;
@@ -1402,7 +1493,7 @@ struct Run {
         pz.distance = step_distance(zstep);
         prof_mark(st, KID_ELEMENTWISE);
         var_pos_prop_table_kernel<<<dim3((unsigned)(WW / EB), (unsigned)Bn), EB, 0, st>>>(
-            tg, pz, pprop, (zstep == 0 && ta.use_edge) ? pprop_edge : nullptr);
+            tg, pz, pprop, (zstep == 0 && ta.use_edge) ? pprop_edge : nullptr, q.fused ? 1.0f / (float)WW : 1.0f);
       };
       if (tilted_prop && !q.per_step) pos_props(0);
       if (var_probe && q.before) {
@@ -1450,7 +1541,45 @@ struct Run {
       // forward multislice (multislice_core.py:61-82)
       // one-pass forward steps: the FP32 engine (at 256 px only where no step spectrum is kept)
       const bool one_pass = q.engine == PTY_DFT_FP32_FFT && !(W == 256 && v && q.inside_grad);
-      for (int z = 0; z < q.Z; ++z) {
+      VarBatch vb{};
+      if (q.fused) {
+        vb.Z = q.Z;
+        vb.Mp = q.Mp;
+        vb.Mo = q.Mo;
+        vb.Bn = Bn;
+        vb.Ny = q.Ny;
+        vb.Nx = q.Nx;
+        vb.use_edge = ta.use_edge;
+        vb.mask_bin = p->smooth_rolloff == 0.0f;
+        vb.pos = d_pos;
+        vb.seq = seq_b;
+        vb.obj = at<float2>(ws, q.o_obj);
+        vb.prop = ta.prop;
+        vb.prop_edge = ta.prop_edge;
+        vb.prop_steps = q.per_step ? steps : nullptr;
+        vb.prop_pos = tilted_prop ? pprop : nullptr;
+        vb.prop_pos_edge = tilted_prop ? pprop_edge : nullptr;
+        vb.mask = ta.mask;
+        vb.mask_sc = ta.mask_sc;
+        vb.sx = ta.sx;
+        vb.tw = fp32_twiddles();
+        vb.obl = ob;
+        vb.stack = stack;
+        vb.gsum = dob;
+        vb.pnat = pbs;     // free between the incoming probe's transform and the probe gradient
+        vb.wnat = psi2;    // free outside the far field
+        vb.fprobe = pb;    // the incoming probe is no longer needed in the adjoint
+        vb.spec = v && q.inside_grad && q.Z > 1 ? spec : nullptr;
+        vb.tilt_w = vb.spec ? at<float>(ws, q.o_tilt_w) : nullptr;
+        vb.tilt_part = at<double>(ws, q.o_tilt_part);
+        vb.px = p->pixel_size_x;
+        vb.py = p->pixel_size_y;
+        vb.err = at<int>(ws, q.o_err);
+        rc = W == 64 ? var_forward<64>(vb, pin, pin_stride == 0, psi, st)
+                     : var_forward<128>(vb, pin, pin_stride == 0, psi, st);
+        if (rc) return rc;
+      }
+      for (int z = 0; z < (q.fused ? 0 : q.Z); ++z) {
         if (z < q.Z - 1 && one_pass) {
           // slice, stack and propagation in one pass (multislice_core.py:61-80); FFT(psi O) kept
           // for the inside-tilt gradient
@@ -1536,7 +1665,22 @@ struct Run {
         }
       }
       // adjoint multislice (multislice_core.py:158-200)
-      for (int z = q.Z - 1; z >= 0; --z) {
+      const bool step_bc = v && v->beam_current && v->step_beam_current;
+      const bool step_ab = v && v->aberrations && v->step_aberrations;
+      const bool step_tb = v && q.before && q.step_tilts;
+      const bool want_probe = p->step_probe || p->step_pos || step_bc || step_ab || step_tb;
+      if (q.fused) {
+        rc = W == 64 ? var_adjoint<64>(vb, psi, p->step_obj != 0, want_probe ? pbs : nullptr, st)
+                     : var_adjoint<128>(vb, psi, p->step_obj != 0, want_probe ? pbs : nullptr, st);
+        if (rc) return rc;
+        if (vb.spec) {
+          // the tables fold 1/W^2 into FFT(g) conj(P)
+          prof_mark(st, KID_ELEMENTWISE);
+          var_inside_sum_kernel<<<(Bn + 127) / 128, 128, 0, st>>>(vb.tilt_part, Bn, nm,
+                                                                  (double)tilt_base * (double)WW, tpart);
+        }
+      }
+      for (int z = q.fused ? -1 : q.Z - 1; z >= 0; --z) {
         prof_mark(st, KID_FUSED);
         adj_slice_kernel<<<grid(q.Mo, Bn), EB, 0, st>>>(psi, stack, ob, dob, z, q.Z, q.Mp, q.Mo, WW);
         if (z > 0) {
@@ -1553,10 +1697,7 @@ struct Run {
                            true, keep);
           if (rc) return rc;
           if (keep) {
-            // sh = -4 pi d / W^2 in float32, d (the step's distance) times the edge multiplier on
-            // the thick step (multislice_core.py:164-180)
-            const float dist = edge ? step_distance(z - 1) * p->edge_mult : step_distance(z - 1);
-            const float shf = fdiv_host((float)-12.566370614359172 * dist, (float)WW);
+            const float shf = tilt_sh(z - 1);
             prof_mark(st, KID_ELEMENTWISE);
             var_inside_tilt_kernel<<<Bn, 1024, 0, st>>>(psi2, spec + (size_t)(z - 1) * spec_stride, nm, W,
                                                         p->pixel_size_x, p->pixel_size_y, (double)shf, tpart);
@@ -1565,22 +1706,21 @@ struct Run {
       }
       if (p->step_obj) {
         // band-limited gradient windows (multislice_core.py:189-191), deterministic scatter
-        if ((rc = band_limit(dob, tmp, (long long)Bn * q.zm))) return rc;
+        if (!q.fused && (rc = band_limit(dob, tmp, (long long)Bn * q.zm))) return rc;
         int* lists = at<int>(ws, q.o_lists);
         int* counts = at<int>(ws, q.o_counts);
         prof_mark(st, KID_TILE_LISTS);
         tile_lists_kernel<<<q.ntiles, 256, 0, st>>>(d_pos, seq_b, Bn, W, q.ntx, lists, counts);
         prof_mark(st, KID_SCATTER);
-        scatter_tiles_kernel<<<dim3(q.ntiles, q.zm), dim3(32, 8), 0, st>>>(
-            dob, d_pos, seq_b, lists, counts, at<float2>(ws, q.o_grad), Bn, W, q.Ny, q.Nx, q.ntx, q.zm, ib > 0);
+        scatter_tiles_kernel<<<dim3(q.ntiles, q.zm, q.sgroups), dim3(32, 8), 0, st>>>(
+            dob, d_pos, seq_b, lists, counts, at<float2>(ws, q.o_grad), Bn, W, q.Ny, q.Nx, q.ntx, q.zm, ib > 0,
+            q.sgroups, q.sgroups > 1 ? at<float2>(ws, q.o_scpart) : nullptr, q.fused ? q.Mp : 1,
+            q.sgroups > 1 ? at<int>(ws, q.o_done) : nullptr);
       }
-      const bool step_bc = v && v->beam_current && v->step_beam_current;
-      const bool step_ab = v && v->aberrations && v->step_aberrations;
-      const bool step_tb = v && q.before && q.step_tilts;
-      if (p->step_probe || p->step_pos || step_bc || step_ab || step_tb) {
+      if (want_probe) {
         // probe-gradient spectra with the shift adjoint and the position gradient (objective.py:641-703)
         prof_mark(st, KID_PROBE_PARTIAL);
-        probe_sum_kernel<<<grid(q.Mp, Bn), EB, 0, st>>>(psi, pbs, q.Mp, q.Mo, WW);
+        if (!q.fused) probe_sum_kernel<<<grid(q.Mp, Bn), EB, 0, st>>>(psi, pbs, q.Mp, q.Mo, WW);
         if ((rc = dft(pbs, pb, (long long)Bn * q.Mp, 0))) return rc;
         prof_mark(st, KID_ELEMENTWISE);
         double* pos_part = at<double>(ws, q.o_pos_part) + (size_t)i0 * q.Mp * 2;
@@ -1636,10 +1776,12 @@ struct Run {
     prof_mark(st, KID_FINALIZE);
     finalize_scalars_kernel<<<1, 256, 0, st>>>(at<double>(ws, q.o_loss_part), at<double>(ws, q.o_pos_part),
                                                at<int>(ws, q.o_seq), q.nseq, q.Mp, W, (double)p->loss_weight,
-                                               p->step_pos && shift, tc_err(), loss_sse, pos_grad);
+                                               p->step_pos && shift, q.fused ? at<int>(ws, q.o_err) : tc_err(),
+                                               loss_sse, pos_grad);
     if (v && q.step_tilts)
-      var_tilt_finalize_kernel<<<1, 32, 0, st>>>(at<double>(ws, q.o_tpart), at<int>(ws, q.o_seq), q.nseq, q.n_rows,
-                                                 q.single_tilt, q.before, q.inside_grad, q.after, v->tilts_grad);
+      var_tilt_finalize_kernel<<<q.single_tilt ? 1 : (q.n_rows + 255) / 256, 256, 0, st>>>(
+          at<double>(ws, q.o_tpart), at<int>(ws, q.o_seq), q.nseq, q.n_rows, q.single_tilt, q.before, q.inside_grad,
+          q.after, v->tilts_grad);
     if (v && q.step_static)
       var_static_final_kernel<<<(WW + 255) / 256, 256, 0, st>>>(at<double>(ws, q.o_sbg), WW,
                                                                v->static_background_grad);

@@ -66,6 +66,8 @@ struct Path {
         (rc = set_smem(fused_multislice_kernel<W, PH_WHOLE>, FusedSmem<W>::bytes)) ||
         (rc = set_smem(fused_multislice_kernel<W, PH_FWD>, FusedSmem<W>::bytes)) ||
         (rc = set_smem(fused_multislice_kernel<W, PH_ADJ>, FusedSmem<W>::bytes)) ||
+        (rc = set_smem(fused_multislice_kernel<W, PH_FWD, true>, FusedSmem<W>::bytes)) ||
+        (rc = set_smem(fused_multislice_kernel<W, PH_ADJ, true>, FusedSmem<W>::bytes)) ||
         (rc = set_smem(grad_windows_kernel<W>, smem)) || (rc = set_smem(probe_final_kernel<W>, smem)))
       return rc;
     return PTY_OK;
@@ -163,7 +165,7 @@ struct Path {
 
   // One launch of the fused kernel's part PH for Bn positions, in clusters of the position's
   // modes where its blocks exchange data.
-  template <int PH>
+  template <int PH, bool TG = false>
   static int launch_fused(const FusedArgs& fa, int Bn, cudaStream_t st) {
     const int nmodes = fa.Mp * fa.Mo;
     const bool clusters = PH == PH_WHOLE || (PH == PH_ADJ && fa.Mo > 1);
@@ -179,7 +181,7 @@ struct Path {
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, fused_multislice_kernel<W, PH>, fa) == cudaSuccess ? PTY_OK : PTY_ERR_CUDA;
+    return cudaLaunchKernelEx(&cfg, fused_multislice_kernel<W, PH, TG>, fa) == cudaSuccess ? PTY_OK : PTY_ERR_CUDA;
   }
 
   // phase 0: the whole pass; 1: forward half (keeps the wave stack, the far field and dL/dI);
@@ -464,6 +466,100 @@ int ms_fused(const MsPlan& q, int step_obj, int step_probe, int use_edge, void* 
   prof_mark(st, KID_FUSED);
   const int rc = Path<W>::template launch_fused<PH>(fa, q.B, st);
   return rc ? rc : cuda_status();
+}
+
+// ------------------------------------------------------------------ variants path
+template <int W>
+FusedArgs var_args(const VarBatch& a) {
+  FusedArgs fa{};
+  fa.Z = a.Z;
+  fa.Mp = a.Mp;
+  fa.Mo = a.Mo;
+  fa.use_edge = a.use_edge;
+  fa.mask_bin = a.mask_bin;
+  fa.loss_weight = 1.0f;
+  fa.obl = a.obl;
+  fa.prop = a.prop;
+  fa.prop_edge = a.prop_edge;
+  fa.prop_steps = a.prop_steps;
+  fa.prop_pos = a.prop_pos;
+  fa.prop_pos_edge = a.prop_pos_edge;
+  fa.pyx = a.prop;          // not used without use_sep
+  fa.mask = a.mask;
+  fa.sx = fa.sy = a.sx;     // not read: the probes come shifted
+  fa.corr = reinterpret_cast<const float*>(a.pos);   // read and not used
+  fa.seq = a.seq;
+  fa.tw = a.tw;
+  fa.stack = a.stack;
+  fa.gsum = a.gsum;
+  fa.fprobe = a.fprobe;
+  fa.spec = a.spec;
+  fa.spec_step = (size_t)a.Bn * a.Mp * a.Mo * W * W;
+  fa.tilt_w = a.tilt_w;
+  fa.tilt_part = a.tilt_part;
+  fa.px = a.px;
+  fa.py = a.py;
+  fa.err = a.err;
+  return fa;
+}
+
+template <int W>
+int var_forward(const VarBatch& a, const float2* probes, bool shared, float2* exit, cudaStream_t st) {
+  constexpr int T = Geo<W>::T;
+  int rc = Path<W>::attributes();
+  if (rc) return rc;
+  WindowArgs wa{};
+  wa.obj = a.obj;
+  wa.pos = a.pos;
+  wa.seq = a.seq;
+  wa.mask_sc = a.mask_sc;
+  wa.tw = a.tw;
+  wa.out = a.obl;
+  wa.Ny = a.Ny;
+  wa.Nx = a.Nx;
+  wa.zm = a.Z * a.Mo;
+  prof_mark(st, KID_OBJECT_WINDOWS);
+  object_windows_kernel<W><<<(unsigned)(a.Bn * a.Z * a.Mo), T, Smem<W>::bytes, st>>>(wa);
+  prof_mark(st, KID_LAYOUT);
+  ref_to_native_kernel<W><<<(shared ? 1 : a.Bn) * a.Mp, T, 0, st>>>(probes, a.pnat, 1, 0);
+  FusedArgs fa = var_args<W>(a);
+  fa.step_obj = 1;
+  fa.probe_b = a.pnat;
+  fa.probe_shared = shared;
+  fa.exit_out = a.wnat;
+  prof_mark(st, KID_FUSED);
+  if ((rc = a.spec ? Path<W>::template launch_fused<PH_FWD, true>(fa, a.Bn, st)
+                   : Path<W>::template launch_fused<PH_FWD>(fa, a.Bn, st)))
+    return rc;
+  prof_mark(st, KID_LAYOUT);
+  native_to_ref_kernel<W><<<a.Bn * a.Mp * a.Mo, T, 0, st>>>(a.wnat, exit, 1, 0);
+  return cuda_status();
+}
+
+template <int W>
+int var_adjoint(const VarBatch& a, const float2* g, bool step_obj, float2* probe_grad, cudaStream_t st) {
+  constexpr int T = Geo<W>::T;
+  int rc = Path<W>::attributes();
+  if (rc) return rc;
+  prof_mark(st, KID_LAYOUT);
+  ref_to_native_kernel<W><<<a.Bn * a.Mp * a.Mo, T, 0, st>>>(g, a.wnat, 1, 0);
+  FusedArgs fa = var_args<W>(a);
+  fa.step_obj = step_obj;
+  fa.step_probe = probe_grad != nullptr;
+  fa.gbuf = a.wnat;
+  prof_mark(st, KID_FUSED);
+  if ((rc = a.spec ? Path<W>::template launch_fused<PH_ADJ, true>(fa, a.Bn, st)
+                   : Path<W>::template launch_fused<PH_ADJ>(fa, a.Bn, st)))
+    return rc;
+  if (step_obj) {
+    prof_mark(st, KID_GRAD_WINDOWS);
+    grad_windows_kernel<W><<<(unsigned)(a.Bn * a.Z * a.Mo), T, Smem<W>::bytes, st>>>(a.gsum, a.mask_sc, a.tw, a.Mp);
+  }
+  if (probe_grad) {
+    prof_mark(st, KID_LAYOUT);
+    native_to_ref_kernel<W><<<a.Bn * a.Mp, T, 0, st>>>(a.fprobe, probe_grad, 1, 0);
+  }
+  return cuda_status();
 }
 
 template <int W>

@@ -255,6 +255,31 @@ struct SideStream {
 };
 int side_stream(SideStream** out);
 
+// The multislice part of one batch of the variants path (64- and 128-px windows, FP32 transforms) on
+// the fused kernel's halves; windows in natural (y, x) order at the boundary.
+struct VarBatch {
+  int Z, Mp, Mo, Bn, Ny, Nx, use_edge, mask_bin;
+  const int *pos, *seq;                 // device: positions (N, 2), the batch's sequence entries
+  const float2 *obj;                    // slice-major object
+  const float2 *prop, *prop_edge, *prop_steps, *prop_pos, *prop_pos_edge;   // scaled by 1/W^2
+  const float *mask, *mask_sc, *sx;
+  float2 *tw, *obl, *stack, *gsum, *pnat, *wnat;   // workspace: twiddles, object windows, waves, gradient
+                                        // contributions, probes and waves in native order
+  float2* fprobe;                       // native probe gradient [Bn*Mp]
+  float2* spec;                         // inside-tilt gradient: step spectra, or nullptr
+  const float* tilt_w;                  // step weights, or nullptr
+  double* tilt_part;                    // [Bn*Mp*Mo][2]
+  float px, py;
+  int* err;
+};
+// probes (natural [Bn*Mp], or [Mp] for all positions with shared) -> exit waves (natural [Bn*Mp*Mo])
+template <int W>
+int var_forward(const VarBatch& a, const float2* probes, bool shared, float2* exit, cudaStream_t st);
+// dL/d(exit wave) (natural) -> gradient windows (natural, window (b, k) at ((b*Z*Mo + k)*Mp) * W^2 of
+// gsum, when step_obj) and the probe gradient summed over object modes (natural [Bn*Mp], when given)
+template <int W>
+int var_adjoint(const VarBatch& a, const float2* g, bool step_obj, float2* probe_grad, cudaStream_t st);
+
 // Launch paths, instantiated in path_w64.cu / path_w128.cu and specialised for W = 256 in
 // path_w256.cu.
 template <int W>

@@ -315,7 +315,8 @@ __global__ void __launch_bounds__(Geo<W>::T) object_windows_kernel(WindowArgs a)
 // ------------------------------------------------------------------ fused multislice
 struct FusedArgs {
   int Z, Mp, Mo, algorithm, step_obj, step_probe, step_pos, probe_shift, simulate, use_edge;
-  const float2* probe_b;    // forward half: given incoming probes, native real [Bb*Mp]; or nullptr
+  const float2* probe_b;    // forward half: given incoming probes, native real [Bb*Mp] (one set [Mp] for
+  int probe_shared;         // all positions with probe_shared); or nullptr
   float2* exit_out;         // forward half: exit waves out instead of the far field, native real [Bb*Mp*Mo]
   float loss_weight;
   const float2* probe;      // (W, W, Mp) reference layout (used without probe shift)
@@ -329,6 +330,16 @@ struct FusedArgs {
                             // the separable shift ramp stand in for the float mask
   const float2* prop_steps; // per-step tables [Z-1] (slice distances), step 0 with the edge
                             // power; nullptr: prop / prop_edge for every step
+  const float2* prop_pos;   // per-position tables [Bb] (tilted propagators) in place of prop, and
+  const float2* prop_pos_edge;   // prop_edge; or nullptr
+  // inside-tilt gradient (kernels with TG): FFT(psi O) of every forward step, native freq [Z-1][Bb*
+  // Mp*Mo], kept by the forward half; the adjoint half sums Im(conj(FFT(psi O)) FFT(g) conj(P)) times
+  // (qy, qx), with each step's weight tilt_w[z], into tilt_part [Bb*Mp*Mo][2]
+  float2* spec;
+  size_t spec_step;         // float2 between steps
+  const float* tilt_w;      // [Z-1], or nullptr: ones
+  double* tilt_part;
+  float px, py;             // pixel sizes (frequencies of the tilt gradient)
   const float* mask;        // natural, unscaled
   const float* sx;
   const float* sy;
@@ -413,6 +424,19 @@ struct FSum {
     return *this;
   }
   __device__ __forceinline__ double value() const { return (double)hi + (double)lo; }
+};
+
+// The same for packs of two terms.
+struct PSum {
+  float2 hi = make_float2(0.f, 0.f), lo = make_float2(0.f, 0.f);
+  __device__ __forceinline__ void add(float2 x) {
+    const float2 s = padd(hi, x), bp = psub(s, hi);
+    lo = padd(lo, padd(psub(hi, psub(s, bp)), psub(x, bp)));
+    hi = s;
+  }
+  __device__ __forceinline__ double value() const {
+    return ((double)hi.x + (double)lo.x) + ((double)hi.y + (double)lo.y);
+  }
 };
 
 // sqrt(x) for x >= 0 and, in r, about 1/sqrt(x): the hardware's reciprocal square root and one step
@@ -522,7 +546,8 @@ struct FusedSmem {
 // per mode.
 enum FusedPart : int { PH_WHOLE = 0, PH_FWD = 1, PH_ADJ = 2 };
 
-template <int W, int PH>
+// TG: with the inside-tilt gradient (multislice_core.py:176-182).
+template <int W, int PH, bool TG = false>
 __global__ void __launch_bounds__(Geo<W>::T, Geo<W>::MINB) fused_multislice_kernel(FusedArgs a) {
   using G = Geo<W>;
   using F = WinFFT<W>;
@@ -651,6 +676,14 @@ __global__ void __launch_bounds__(Geo<W>::T, Geo<W>::MINB) fused_multislice_kern
     }
   };
 
+  // the shared or the position's propagator of the step from slice z to z + 1
+  auto prop_table = [&](int z) -> const float2* {
+    const bool edge = z == 0 && a.use_edge;
+    if (PH != PH_WHOLE && a.prop_pos) return (edge ? a.prop_pos_edge : a.prop_pos) + (size_t)b * WW;
+    return a.prop_steps ? a.prop_steps + (size_t)z * WW : (edge ? a.prop_edge : a.prop);
+  };
+
+  PSum tgy, tgx;   // TG: the tilt gradient's sums
   Win v;
   int side_next = -1;        // the slice whose window prefix the side buffer takes next
   bool side_held = false;    // the side buffer holds the next step's operand, waited for
@@ -674,7 +707,7 @@ __global__ void __launch_bounds__(Geo<W>::T, Geo<W>::MINB) fused_multislice_kern
     if (far_start) {
     } else if (PH != PH_ADJ && s == 0) {
       if (PH == PH_FWD && a.probe_b) {
-        ld_native(a.probe_b + ((size_t)b * a.Mp + p) * WW, v);
+        ld_native(a.probe_b + ((a.probe_shared ? 0 : (size_t)b * a.Mp) + p) * WW, v);
       } else if (!a.probe_shift) {
 #pragma unroll
         for (int i = 0; i < 32; ++i) wset(v, i, a.probe[(size_t)(G::ry(t) * W + G::rx(t, i)) * a.Mp + p]);
@@ -823,12 +856,11 @@ __global__ void __launch_bounds__(Geo<W>::T, Geo<W>::MINB) fused_multislice_kern
         }
       }
     } else if (PH != PH_ADJ && fwd && z < Z - 1) {
+      if constexpr (TG) st_native(a.spec + (size_t)z * a.spec_step + (size_t)blockIdx.x * WW, v);
       if (a.use_sep && !(z == 0 && a.use_edge)) {
         propagate_sep(v, false);
       } else {
-        const float2* pr = a.prop_steps ? a.prop_steps + (size_t)z * WW
-                                        : ((z == 0 && a.use_edge) ? a.prop_edge : a.prop);
-        mul_table<W>(v, pr, false);
+        mul_table<W>(v, prop_table(z), false);
       }
     } else if (PH == PH_FWD && fwd) {
       // far field: Psi = FFT(exit) * mask (objective.py:501-503); far_field_loss_kernel goes on
@@ -952,9 +984,25 @@ __global__ void __launch_bounds__(Geo<W>::T, Geo<W>::MINB) fused_multislice_kern
       if (a.use_sep && !(z == 1 && a.use_edge)) {
         propagate_sep(v, true);
       } else {
-        const float2* pr = a.prop_steps ? a.prop_steps + (size_t)(z - 1) * WW
-                                        : ((z == 1 && a.use_edge) ? a.prop_edge : a.prop);
-        mul_table<W>(v, pr, true);
+        mul_table<W>(v, prop_table(z - 1), true);
+      }
+      if constexpr (TG) {
+        const float4* f4 = reinterpret_cast<const float4*>(a.spec + (size_t)(z - 1) * a.spec_step +
+                                                           (size_t)blockIdx.x * WW) + wo;
+        const float2 w = pdup(a.tilt_w ? a.tilt_w[z - 1] : 1.0f);
+#pragma unroll
+        for (int q = 0; q < G::Q / 2; ++q) {
+          const int kx = G::fkx(t, 2 * q * G::Bq);
+          const float2 qx = pmul(make_float2(fftfreq_f32(kx, W, a.px), fftfreq_f32(kx + W / 2, W, a.px)), w);
+#pragma unroll
+          for (int r = 0; r < G::Bq; ++r) {
+            const int j = q * G::Bq + r;
+            const float4 f = f4[j * 32];
+            const float2 im = psub(pmul(make_float2(f.x, f.y), v.im[j]), pmul(make_float2(f.z, f.w), v.re[j]));
+            tgx.add(pmul(qx, im));
+            tgy.add(pmul(pmul(pdup(fftfreq_f32(G::fky(t, 2 * j), W, a.py)), w), im));
+          }
+        }
       }
     } else if (PH != PH_FWD) {
       // probe-gradient spectrum with the shift adjoint, position gradient (objective.py:641-656)
@@ -1041,6 +1089,14 @@ __global__ void __launch_bounds__(Geo<W>::T, Geo<W>::MINB) fused_multislice_kern
     F::inverse_tail(v);
   }
   if (lane == 0) bulk_wait_all();   // the bulk stores are complete before the block exits
+  if constexpr (TG && PH == PH_ADJ) {
+    double gy = tgy.value(), gx = tgx.value();
+    block_sum2(gy, gx, red);
+    if (t == 0) {
+      a.tilt_part[2 * (size_t)blockIdx.x] = gy;
+      a.tilt_part[2 * (size_t)blockIdx.x + 1] = gx;
+    }
+  }
 }
 
 // ------------------------------------------------------------------ loss of the halves
