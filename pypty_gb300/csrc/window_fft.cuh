@@ -30,10 +30,10 @@
 // transform.
 //
 // Packed arithmetic. The window is held as 16 packs of two values, real and imaginary parts
-// apart (struct Win), and nearly all of the arithmetic is two-wide (add/mul/fma.f32x2): the
-// kernels are bound by instruction issue, and a packed instruction does two lanes' work in one
-// issue slot. The two halves of a pack go through the same butterflies: round 1 packs the even
-// and odd x of a 16-point DFT each (a scalar radix-2 stage joins them), round 2 packs
+// apart (struct Win), and nearly all of the arithmetic is two-wide (add/mul/fma.f32x2): a packed
+// instruction does two lanes' work in one issue slot. The two halves of a pack go through the same
+// butterflies: round 1 packs the even and odd x of a 16-point DFT each (a scalar radix-2 stage
+// joins them; the inverse the even and odd k), round 2 packs
 // neighbouring n2, round 3 packs kx and kx + W/2. The exchanges store 16-byte words of real and
 // imaginary packs, so that loads give packs without register moves.
 //
@@ -285,6 +285,68 @@ __device__ __forceinline__ void ptw(float2& re, float2& im) {
   }
 }
 
+// one and two-wide FP32 under the same names
+__device__ __forceinline__ float vadd(float a, float b) { return a + b; }
+__device__ __forceinline__ float vsub(float a, float b) { return a - b; }
+__device__ __forceinline__ float vfma(float a, float b, float c) { return fmaf(a, b, c); }
+__device__ __forceinline__ float2 vadd(float2 a, float2 b) { return padd(a, b); }
+__device__ __forceinline__ float2 vsub(float2 a, float2 b) { return psub(a, b); }
+__device__ __forceinline__ float2 vfma(float2 a, float b, float2 c) { return pfma(a, pdup(b), c); }
+
+// (s, d) = (a + w b, a - w b), w = exp(SIGN * 2 pi i E / N): the twiddle's products fuse with the
+// butterfly's adds, one rounding less than multiplying first, for the same number of instructions
+// (two fewer at odd multiples of pi/4)
+template <int N, int E, int SIGN, typename V>
+__device__ __forceinline__ void add_sub_tw(V ar, V ai, V br, V bi, V& sr, V& si, V& dr, V& di) {
+  constexpr int m = ((E % N) * (32 / N)) & 31;
+  if constexpr (m % 8 == 0) {                 // w = 1, +-i, -1
+    constexpr bool swap = m % 16 == 8;
+    constexpr bool neg_r = swap ? ((m == 8) == (SIGN > 0)) : m == 16;      // w b = (-+bi, +-br) or -b
+    constexpr bool neg_i = swap ? !neg_r : m == 16;
+    const V wr = swap ? bi : br, wi = swap ? br : bi;
+    sr = neg_r ? vsub(ar, wr) : vadd(ar, wr);
+    si = neg_i ? vsub(ai, wi) : vadd(ai, wi);
+    dr = neg_r ? vadd(ar, wr) : vsub(ar, wr);
+    di = neg_i ? vadd(ai, wi) : vsub(ai, wi);
+  } else if constexpr (m % 4 == 0) {          // c (1 + i t), |c| = sqrt(1/2), t = +-1
+    constexpr float h = 7.071067691e-01f;
+    constexpr float c = kcos32(m) > 0 ? h : -h;
+    constexpr float s = (SIGN > 0 ? 1.0f : -1.0f) * (ksin32(m) > 0 ? h : -h);
+    constexpr bool same = (c > 0) == (s > 0);
+    const V u = same ? vsub(br, bi) : vadd(br, bi);
+    const V w = same ? vadd(bi, br) : vsub(bi, br);
+    sr = vfma(u, c, ar);
+    si = vfma(w, c, ai);
+    dr = vfma(u, -c, ar);
+    di = vfma(w, -c, ai);
+  } else {
+    constexpr float c = kcos32(m);
+    constexpr float s = (SIGN > 0 ? 1.0f : -1.0f) * ksin32(m);
+    sr = vfma(br, c, vfma(bi, -s, ar));
+    si = vfma(bi, c, vfma(br, s, ai));
+    dr = vfma(br, -c, vfma(bi, s, ar));
+    di = vfma(bi, -c, vfma(br, -s, ai));
+  }
+}
+
+// 4-point butterfly of (t0, w^e t1, w^2e t2, w^3e t3), w = exp(SIGN * 2 pi i / N)
+template <int N, int E, int SIGN>
+__device__ __forceinline__ void pbfly4_tw(float2& r0, float2& i0, float2& r1, float2& i1, float2& r2, float2& i2,
+                                          float2& r3, float2& i3) {
+  float2 ur0, ui0, ur1, ui1, ur2, ui2, dr, di;
+  add_sub_tw<N, 2 * E, SIGN>(r0, i0, r2, i2, ur0, ui0, ur1, ui1);
+  ptw<N, E, SIGN>(r1, i1);
+  add_sub_tw<N, 3 * E, SIGN>(r1, i1, r3, i3, ur2, ui2, dr, di);
+  r0 = padd(ur0, ur2);
+  i0 = padd(ui0, ui2);
+  r2 = psub(ur0, ur2);
+  i2 = psub(ui0, ui2);
+  r1 = SIGN > 0 ? psub(ur1, di) : padd(ur1, di);
+  i1 = SIGN > 0 ? padd(ui1, dr) : psub(ui1, dr);
+  r3 = SIGN > 0 ? padd(ur1, di) : psub(ur1, di);
+  i3 = SIGN > 0 ? psub(ui1, dr) : padd(ui1, dr);
+}
+
 template <int SIGN>
 __device__ __forceinline__ void pbfly4(float2& r0, float2& i0, float2& r1, float2& i1, float2& r2, float2& i2,
                                        float2& r3, float2& i3) {
@@ -328,10 +390,7 @@ struct PDFT {
         float2 r1 = re[OFF + STRIDE * (4 * k + 1)], i1 = im[OFF + STRIDE * (4 * k + 1)];
         float2 r2 = re[OFF + STRIDE * (4 * k + 2)], i2 = im[OFF + STRIDE * (4 * k + 2)];
         float2 r3 = re[OFF + STRIDE * (4 * k + 3)], i3 = im[OFF + STRIDE * (4 * k + 3)];
-        ptw<N, 1 * k, SIGN>(r1, i1);
-        ptw<N, 2 * k, SIGN>(r2, i2);
-        ptw<N, 3 * k, SIGN>(r3, i3);
-        pbfly4<SIGN>(r0, i0, r1, i1, r2, i2, r3, i3);
+        pbfly4_tw<N, k, SIGN>(r0, i0, r1, i1, r2, i2, r3, i3);
         outr[k] = r0, outi[k] = i0;
         outr[k + M] = r1, outi[k + M] = i1;
         outr[k + 2 * M] = r2, outi[k + 2 * M] = i2;
@@ -398,9 +457,8 @@ struct WinFFT {
     PDFT<16, -1>::template run<1, 0>(v.re, v.im);
     static_for<0, 16>([&](auto KK) {
       constexpr int k = decltype(KK)::value;
-      const float2 o = tw<32, k, -1>(make_float2(v.re[k].y, v.im[k].y));
-      const float2 e = make_float2(v.re[k].x, v.im[k].x);
-      const float2 a = cadd(e, o), b = csub(e, o);
+      float2 a, b;
+      add_sub_tw<32, k, -1>(v.re[k].x, v.im[k].x, v.re[k].y, v.im[k].y, a.x, a.y, b.x, b.y);
       // row k1, word (lane / 4) ^ (k1 & 7); rows k and k + 16 share the swizzle
       float* d = xw + k * 32 + ((((lane >> 2) ^ (k & 7)) << 2) | (lane & 3));
       d[0] = a.x;
@@ -484,7 +542,18 @@ struct WinFFT {
   // The register-only end of the inverse transform (round 1): callers that reuse xbuf may
   // run inverse_head (everything up to the last xbuf read), __syncwarp, refill the warp's part
   // of xbuf asynchronously, and then run inverse_tail while the copy is in flight.
-  static __device__ __forceinline__ void inverse_tail(Win& v) { PDFT<16, +1>::template run<1, 0>(v.re, v.im); }
+  static __device__ __forceinline__ void inverse_tail(Win& v) {
+    // 16-point DFTs of the even and odd k, then x_n, x_{n+16} = E_n +- w_32^-n O_n
+    PDFT<16, +1>::template run<1, 0>(v.re, v.im);
+    Win e = v;
+    static_for<0, 16>([&](auto NN) {
+      constexpr int n = decltype(NN)::value;
+      float2 a, b;
+      add_sub_tw<32, n, +1>(e.re[n].x, e.im[n].x, e.re[n].y, e.im[n].y, a.x, a.y, b.x, b.y);
+      wset(v, n, a);
+      wset(v, n + 16, b);
+    });
+  }
 
   // inverse() without its register-only tail
   static __device__ __forceinline__ void inverse_head(Win& v, float2* xbuf, const float2* tw1, const float2* tw2) {
@@ -553,13 +622,13 @@ struct WinFFT {
       }
     }
     __syncwarp();
-    static_for<0, 16>([&](auto KK) {
-      constexpr int k = decltype(KK)::value;
-      const float* d = xw + k * 32 + ((((lane >> 2) ^ (k & 7)) << 2) | (lane & 3));
-      const float2 a = make_float2(d[0], d[PLANE]), b = make_float2(d[16 * 32], d[16 * 32 + PLANE]);
-      const float2 e = cadd(a, b), o = tw<32, k, +1>(csub(a, b));
-      v.re[k] = make_float2(e.x, o.x);
-      v.im[k] = make_float2(e.y, o.y);
+    // pack m: the elements k = 2m and 2m + 1 of this lane's row
+    static_for<0, 16>([&](auto MM) {
+      constexpr int m = decltype(MM)::value, k = 2 * m;
+      const float* d0 = xw + k * 32 + ((((lane >> 2) ^ (k & 7)) << 2) | (lane & 3));
+      const float* d1 = xw + (k + 1) * 32 + ((((lane >> 2) ^ ((k + 1) & 7)) << 2) | (lane & 3));
+      v.re[m] = make_float2(d0[0], d1[0]);
+      v.im[m] = make_float2(d0[PLANE], d1[PLANE]);
     });
   }
 };
