@@ -10,10 +10,48 @@
 #pragma once
 #include "plan.h"
 #include "ptycho_kernels.cuh"
+#include "window_stream.cuh"
 
 namespace pty {
 
 static_assert(TS == kTileSize, "scatter tile size of the kernels and the plan");
+
+// Windows per block of the streaming passes: a block loads its first window with nothing to hide
+// the load under (about half a window's time), and the waves of blocks should end full.
+inline int stream_run(int n) {
+  int best = 1;
+  long long best_cost = 0;
+  for (int run = 1; run <= 16; ++run) {
+    const long long blocks = (n + run - 1) / run;
+    const long long cost = (blocks + kSMs - 1) / kSMs * (2 * run + 1);
+    if (run == 1 || cost < best_cost) best = run, best_cost = cost;
+  }
+  return best;
+}
+
+// band-limited object windows / gradient windows, n of them
+template <int W>
+int launch_object_windows(const WindowArgs& wa, int n, cudaStream_t st) {
+  if constexpr (W == 128) {
+    const int run = stream_run(n);
+    object_windows_stream_kernel<<<(unsigned)((n + run - 1) / run), Geo<W>::T, Stream128::bytes, st>>>(wa, n, run);
+  } else {
+    object_windows_kernel<W><<<(unsigned)n, Geo<W>::T, Smem<W>::bytes, st>>>(wa);
+  }
+  return cuda_status();
+}
+
+template <int W>
+int launch_grad_windows(float2* buf, const float* mask_sc, const float2* tw, int nsum, int n, cudaStream_t st) {
+  if constexpr (W == 128) {
+    const int run = stream_run(n);
+    grad_windows_stream_kernel<<<(unsigned)((n + run - 1) / run), Geo<W>::T, Stream128::bytes, st>>>(buf, mask_sc, tw,
+                                                                                                 nsum, n, run);
+  } else {
+    grad_windows_kernel<W><<<(unsigned)n, Geo<W>::T, Smem<W>::bytes, st>>>(buf, mask_sc, tw, nsum);
+  }
+  return cuda_status();
+}
 
 template <int W>
 struct Path {
@@ -62,14 +100,21 @@ struct Path {
   static int attributes() {
     const size_t smem = Smem<W>::bytes;
     int rc;
-    if ((rc = set_smem(probe_fft_kernel<W>, smem)) || (rc = set_smem(object_windows_kernel<W>, smem)) ||
+    if ((rc = set_smem(probe_fft_kernel<W>, smem)) ||
         (rc = set_smem(fused_multislice_kernel<W, PH_WHOLE>, FusedSmem<W>::bytes)) ||
         (rc = set_smem(fused_multislice_kernel<W, PH_FWD>, FusedSmem<W>::bytes)) ||
         (rc = set_smem(fused_multislice_kernel<W, PH_ADJ>, FusedSmem<W>::bytes)) ||
         (rc = set_smem(fused_multislice_kernel<W, PH_FWD, true>, FusedSmem<W>::bytes)) ||
         (rc = set_smem(fused_multislice_kernel<W, PH_ADJ, true>, FusedSmem<W>::bytes)) ||
-        (rc = set_smem(grad_windows_kernel<W>, smem)) || (rc = set_smem(probe_final_kernel<W>, smem)))
+        (rc = set_smem(probe_final_kernel<W>, smem)))
       return rc;
+    if constexpr (W == 128) {
+      if ((rc = set_smem(object_windows_stream_kernel, Stream128::bytes)) ||
+          (rc = set_smem(grad_windows_stream_kernel, Stream128::bytes)))
+        return rc;
+    } else {
+      if ((rc = set_smem(object_windows_kernel<W>, smem)) || (rc = set_smem(grad_windows_kernel<W>, smem))) return rc;
+    }
     return PTY_OK;
   }
 
@@ -159,8 +204,7 @@ struct Path {
     wa.Nx = q.Nx;
     wa.zm = q.zm;
     prof_mark(side, KID_OBJECT_WINDOWS);
-    object_windows_kernel<W><<<(unsigned)(batch_count(ib) * q.zm), T, Smem<W>::bytes, side>>>(wa);
-    return cuda_status();
+    return launch_object_windows<W>(wa, batch_count(ib) * q.zm, side);
   }
 
   // One launch of the fused kernel's part PH for Bn positions, in clusters of the position's
@@ -250,7 +294,8 @@ struct Path {
       float2* gs = gsum(ib);
       float2* gdst = grad_out ? grad_out : at<float2>(ws, q.o_grad);
       prof_mark(side, KID_GRAD_WINDOWS);
-      grad_windows_kernel<W><<<(unsigned)(Bn * q.zm), T, Smem<W>::bytes, side>>>(gs, ta.mask_sc, tw, q.Mp);
+      int rc = launch_grad_windows<W>(gs, ta.mask_sc, tw, q.Mp, Bn * q.zm, side);
+      if (rc) return rc;
       int* lists = at<int>(ws, q.o_lists);
       int* counts = at<int>(ws, q.o_counts);
       if (!lists_done) {
@@ -519,7 +564,7 @@ int var_forward(const VarBatch& a, const float2* probes, bool shared, float2* ex
   wa.Nx = a.Nx;
   wa.zm = a.Z * a.Mo;
   prof_mark(st, KID_OBJECT_WINDOWS);
-  object_windows_kernel<W><<<(unsigned)(a.Bn * a.Z * a.Mo), T, Smem<W>::bytes, st>>>(wa);
+  if ((rc = launch_object_windows<W>(wa, a.Bn * a.Z * a.Mo, st))) return rc;
   prof_mark(st, KID_LAYOUT);
   ref_to_native_kernel<W><<<(shared ? 1 : a.Bn) * a.Mp, T, 0, st>>>(probes, a.pnat, 1, 0);
   FusedArgs fa = var_args<W>(a);
@@ -553,7 +598,7 @@ int var_adjoint(const VarBatch& a, const float2* g, bool step_obj, float2* probe
     return rc;
   if (step_obj) {
     prof_mark(st, KID_GRAD_WINDOWS);
-    grad_windows_kernel<W><<<(unsigned)(a.Bn * a.Z * a.Mo), T, Smem<W>::bytes, st>>>(a.gsum, a.mask_sc, a.tw, a.Mp);
+    if ((rc = launch_grad_windows<W>(a.gsum, a.mask_sc, a.tw, a.Mp, a.Bn * a.Z * a.Mo, st))) return rc;
   }
   if (probe_grad) {
     prof_mark(st, KID_LAYOUT);
@@ -619,8 +664,8 @@ int run_ms_grads(const MsPlan& q, const float2* d_exit, const float2* waves, con
     float2* grad = at<float2>(ws, q.o_grad);
     const int nyx = q.Ny * q.Nx;
     prof_mark(st, KID_GRAD_WINDOWS);
-    grad_windows_kernel<W><<<(unsigned)(q.B * q.zm), T, Smem<W>::bytes, st>>>(gs, at<float>(ws, q.o_mask_sc),
-                                                                            at<float2>(ws, q.o_tw), q.Mp);
+    if ((rc = launch_grad_windows<W>(gs, at<float>(ws, q.o_mask_sc), at<float2>(ws, q.o_tw), q.Mp, q.B * q.zm, st)))
+      return rc;
     prof_mark(st, KID_OBJ_TO_SLICES);
     obj_to_slices_kernel<<<(nyx + 255) / 256, 256, 0, st>>>(object_grad, grad, nyx, q.zm);
     prof_mark(st, KID_TILE_LISTS);
@@ -668,13 +713,21 @@ int run_scatteradd(const MsPlan& q, float2* full, const float2* chop, void* ws, 
 template <int W>
 int run_fft2(const float2* in, float2* out, int batch, int inverse, int shift, float2* tw, cudaStream_t st,
              int build_tw) {
-  if (set_smem(fft2_batch_kernel<W>, Smem<W>::bytes)) return PTY_ERR_CUDA;
   if (build_tw) {
     prof_mark(st, KID_TWIDDLES);
     build_twiddles_kernel<W><<<1, 256, 0, st>>>(tw);
   }
   prof_mark(st, KID_FFT2);
-  fft2_batch_kernel<W><<<batch, Geo<W>::T, Smem<W>::bytes, st>>>(in, out, inverse, shift, tw);
+  if constexpr (W == 128) {
+    auto kernel = inverse ? (shift ? fft2_stream_kernel<1, 64> : fft2_stream_kernel<1, 0>)
+                          : (shift ? fft2_stream_kernel<0, 64> : fft2_stream_kernel<0, 0>);
+    if (set_smem(kernel, Stream128::bytes)) return PTY_ERR_CUDA;
+    const int run = stream_run(batch);
+    kernel<<<(unsigned)((batch + run - 1) / run), Geo<W>::T, Stream128::bytes, st>>>(in, out, batch, run, tw);
+  } else {
+    if (set_smem(fft2_batch_kernel<W>, Smem<W>::bytes)) return PTY_ERR_CUDA;
+    fft2_batch_kernel<W><<<batch, Geo<W>::T, Smem<W>::bytes, st>>>(in, out, inverse, shift, tw);
+  }
   prof_mark(st, -1);
   return cuda_status();
 }
