@@ -47,8 +47,8 @@ constexpr int kSMs = 152;
 // blocks the scatter aims for: two per SM
 constexpr int kScatterBlocks = 2 * kSMs;
 
-// blocks of the fused kernel that the GPU holds at once (64-px windows: two per SM)
-constexpr int resident_blocks(int W) { return W == 64 ? 2 * kSMs : kSMs; }
+// blocks of the fused kernel that the GPU holds at once (64-px windows: three per SM)
+constexpr int resident_blocks(int W) { return W == 64 ? 3 * kSMs : kSMs; }
 
 // twiddle tables in global memory: W = 256 windows use the 128 tables of their sub-transforms
 inline int tw_count(int W) { return W == 64 ? Geo<64>::TW1 + Geo<64>::TW2 : Geo<128>::TW1 + Geo<128>::TW2; }
@@ -135,8 +135,8 @@ inline Plan make_plan(const pty_problem_t* p, bool split = false) {
   // several modes and about fills the GPU. The halves use the SMs that clusters leave idle and
   // form the loss once per position, for two more launches (~10 us of a call). Whole pass against
   // halves: 128 px, 768 blocks x 20 slices, four batches, 18.4 -> 16.4 ms; 128 blocks x 7 slices,
-  // three batches, 1036 -> 1004 us; 108 blocks x 3 slices 248 -> 251 us; 64 px, 768 blocks x 6
-  // slices 563 -> 522 us; 256 blocks x 8 slices 277 -> 286 us.
+  // three batches, 1036 -> 1004 us; 108 blocks x 3 slices 248 -> 251 us; 64 px, 1200 blocks x 8
+  // slices 802 -> 727 us, 480 x 6 365 -> 349 us, 440 x 6 278 -> 283 us, 400 x 1 98 -> 110 us.
   const int blocks = q.Bb * q.Mp;
   q.halves = !w256 && !split && q.Mo == 1 && q.Mp > 1 && blocks > (q.W == 64 ? resident_blocks(64) : kSMs * 3 / 4);
   const bool far = w256 || split || q.halves;

@@ -375,33 +375,25 @@ __device__ __forceinline__ float2 shift_ramp(const FusedArgs& a, int ky, int kx,
   return make_float2(c * mk, s * mk);
 }
 
-// The same ramp for a binary mask, inside the mask: exp(i sx[kx] dx) * exp(i sy[ky] dy). A
-// thread's 32 frequency-layout elements span Q distinct kx and Bq distinct ky, so Q + Bq sincos
-// evaluations serve all 32 (the caller zeroes the elements outside the mask). f(i, ky, kx, ramp)
-// is called for every element, i a compile-time constant.
+// The same ramp for a binary mask, inside the mask: exp(i sx[kx] dx) * exp(i sy[ky] dy), from a table of
+// both factors (y, then x; 2 W entries) that the block forms once in shared memory. f(j, ky, kx, re, im)
+// is called for every pack, (re, im) its two elements' ramps, kx and kx + W/2.
 template <int W, typename Fn>
-__device__ __forceinline__ void visit_sep_ramp(const FusedArgs& a, int t, float dy, float dx, Fn&& f) {
+__device__ __forceinline__ void visit_sep_ramp(const float2* table, int t, Fn&& f) {
   using G = Geo<W>;
-  constexpr int Q = G::Q, Bq = G::Bq;
-  auto phase = [](float s, float d) {
-    float sn, cs;
-    sincosf(__fmul_rn(s, d), &sn, &cs);
-    return make_float2(cs, sn);
-  };
-  float2 ey[Bq];
-  static_for<0, Bq>([&](auto RR) {
-    constexpr int r = decltype(RR)::value;
-    ey[r] = phase(a.sy[G::fky(t, 2 * r)], dy);
-  });
-  static_for<0, Q>([&](auto QQ) {   // kx number q: half q % 2 of the packs (q / 2) * Bq + r
-    constexpr int q = decltype(QQ)::value, i0 = 2 * (q / 2) * Bq + q % 2;
-    const int kx = G::fkx(t, i0);
-    const float2 ex = phase(a.sx[kx], dx);
-    static_for<0, Bq>([&](auto RR) {
-      constexpr int i = i0 + 2 * decltype(RR)::value;
-      f(std::integral_constant<int, i>{}, G::fky(t, i), kx, cmul(ex, ey[decltype(RR)::value]));
-    });
-  });
+#pragma unroll
+  for (int q = 0; q < G::Q / 2; ++q) {
+    const int kx = G::fkx(t, 2 * q * G::Bq);
+    const float2 xa = table[W + kx], xb = table[W + kx + W / 2];
+    const float2 xr = make_float2(xa.x, xb.x), xi = make_float2(xa.y, xb.y), nxi = pneg(xi);
+#pragma unroll
+    for (int r = 0; r < G::Bq; ++r) {
+      const int j = q * G::Bq + r, ky = G::fky(t, 2 * j);
+      const float2 y = table[ky];
+      const float2 yr = pdup(y.x), yi = pdup(y.y);
+      f(j, ky, kx, pfma(yi, nxi, pmul(yr, xr)), pfma(yi, xr, pmul(yr, xi)));
+    }
+  }
 }
 
 // Detector (fftshifted) pixel of element i of thread t in the frequency layout.
@@ -506,11 +498,12 @@ struct FusedSmem {
   static constexpr size_t pyx_off = side_off + sizeof(float2) * NST * Geo<W>::T;
   static constexpr size_t bits_off = pyx_off + sizeof(float2) * 3 * W;   // y factors as packs, x factors
   static constexpr size_t bar_off = bits_off + sizeof(uint32_t) * Geo<W>::T;
-  // W = 64: the position's measured pattern (W^2 floats, detector order), copied in at the
-  // start, and the probe-shift ramp of the first step (frequency layout), reused by the last
-  static constexpr size_t meas_off = (bar_off + 2 * (Geo<W>::T / 32) * sizeof(uint64_t) + 15) & ~(size_t)15;
-  static constexpr size_t ramp_off = meas_off + (W == 64 ? sizeof(float) * W * W : 0);
-  static constexpr size_t bytes = ramp_off + (W == 64 ? sizeof(float2) * W * W : 0);
+  // the probe shift's phase factors along y and x (binary mask), for the first step and the last
+  static constexpr size_t phase_off = bar_off + 2 * (Geo<W>::T / 32) * sizeof(uint64_t);
+  // W = 64: the position's measured pattern (W^2 floats, detector order), copied in at the start
+  static constexpr size_t meas_off = (phase_off + sizeof(float2) * 2 * W + 15) & ~(size_t)15;
+  static constexpr size_t bytes = meas_off + (W == 64 ? sizeof(float) * W * W : 0);
+  static_assert(bytes <= 232448, "shared memory of a block");
 };
 
 // One thread block per (position, probe mode, object mode); the Mp*Mo blocks of a position
@@ -555,10 +548,9 @@ __global__ void __launch_bounds__(Geo<W>::T, Geo<W>::MINB) fused_multislice_kern
   constexpr int T = G::T;
   constexpr int NST = S::NST;
   constexpr size_t WW = (size_t)W * W;
-  // W = 64 (few slices, latency-bound far field and probe steps): mask bits instead of the
-  // float mask, the separable shift ramp, the measured pattern copied into shared memory at the
-  // start. At W = 128 the extra live values spill and shared memory is full, so these stay
-  // compiled out there.
+  // W = 64 (few slices, latency-bound far field): mask bits instead of the float mask, the measured
+  // pattern copied into shared memory at the start. At W = 128 the extra live values spill and
+  // shared memory is full, so these stay compiled out there.
   constexpr bool kLean = (W == 64);
   extern __shared__ __align__(16) unsigned char smem[];
   float2 *xbuf, *tw1, *tw2;
@@ -599,6 +591,17 @@ __global__ void __launch_bounds__(Geo<W>::T, Geo<W>::MINB) fused_multislice_kern
     spy[i] = make_float4(y.x, y.x, y.y, y.y);
     spx[i] = a.pyx[W + i];
   }
+  // Every thread forming its own elements' factors (18 sincosf each, inlined) held the first step of
+  // 128-px blocks for 35k cycles and the last for 48k, against 26k for a slice; with 2 W of them per
+  // block these take 5k and 19k.
+  float2* sph = reinterpret_cast<float2*>(smem + S::phase_off);
+  if (a.probe_shift && a.mask_bin) {
+    for (int i = t; i < 2 * W; i += T) {
+      float sn, cs;
+      sincosf(i < W ? __fmul_rn(a.sy[i], dy) : __fmul_rn(a.sx[i - W], dx), &sn, &cs);
+      sph[i] = make_float2(cs, sn);
+    }
+  }
   // bit i: element i (frequency layout) of this thread lies inside the band limit
   {
     uint32_t mbits = 0;
@@ -608,7 +611,6 @@ __global__ void __launch_bounds__(Geo<W>::T, Geo<W>::MINB) fused_multislice_kern
   }
   __syncthreads();
   float* smeas = reinterpret_cast<float*>(smem + S::meas_off);    // W = 64 only
-  float2* sramp = reinterpret_cast<float2*>(smem + S::ramp_off);  // W = 64 only
   if constexpr (kLean) {
     // only passes that reach the far field (which waits for these copies) issue them
     if (PH == PH_WHOLE && !a.simulate && a.measured) {
@@ -673,6 +675,17 @@ __global__ void __launch_bounds__(Geo<W>::T, Geo<W>::MINB) fused_multislice_kern
         v.re[j] = make_float2(in0 ? v.re[j].x : 0.f, in1 ? v.re[j].y : 0.f);
         v.im[j] = make_float2(in0 ? v.im[j].x : 0.f, in1 ? v.im[j].y : 0.f);
       }
+    }
+  };
+
+  // a rolled-off mask's ramp, element i of thread t at i * T + t. A loop of its own, because inlined
+  // for each of the window's registers sincosf does not fit the instruction cache (first step of
+  // 128-px blocks 46k cycles, last 69k; now 23k and 47k).
+  auto ramp_to_xbuf = [&]() {
+#pragma unroll 4
+    for (int i = 0; i < 32; ++i) {
+      const int ky = G::fky(t, i), kx = G::fkx(t, i);
+      xbuf[i * T + t] = shift_ramp<W>(a, ky, kx, a.mask[ky * W + kx], dy, dx);
     }
   };
 
@@ -842,18 +855,19 @@ __global__ void __launch_bounds__(Geo<W>::T, Geo<W>::MINB) fused_multislice_kern
       const float inv = 1.0f / (float)WW;
       if (a.mask_bin) {
         const uint32_t mbits = sbits[t];
-        ld_native(pf, v);   // all loads in flight before the ramps are formed
-        visit_sep_ramp<W>(a, t, dy, dx, [&](auto I, int, int, float2 ramp) {
-          constexpr int i = decltype(I)::value;
-          if constexpr (PH == PH_WHOLE && kLean) sramp[i * T + t] = ramp;   // serves the probe-gradient step too
-          wset(v, i, ((mbits >> i) & 1u) ? cscale(cmul(wget(v, i), ramp), inv) : make_float2(0.f, 0.f));
+        ld_native(pf, v);
+        visit_sep_ramp<W>(sph, t, [&](int j, int, int, float2 rr, float2 ri) {
+          pcmul(v.re[j], v.im[j], rr, ri, pneg(ri));
+          const float s0 = ((mbits >> (2 * j)) & 1u) ? inv : 0.f, s1 = ((mbits >> (2 * j + 1)) & 1u) ? inv : 0.f;
+          v.re[j] = pmul(v.re[j], make_float2(s0, s1));
+          v.im[j] = pmul(v.im[j], make_float2(s0, s1));
         });
       } else {
+        ramp_to_xbuf();
+        ld_native(pf, v);
 #pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          const int ky = G::fky(t, i), kx = G::fkx(t, i);
-          wset(v, i, cscale(cmul(native_at(pf, i, t), shift_ramp<W>(a, ky, kx, a.mask[ky * W + kx], dy, dx)), inv));
-        }
+        for (int i = 0; i < 32; ++i) wset(v, i, cscale(cmul(wget(v, i), xbuf[i * T + t]), inv));
+        __syncthreads();   // the inverse transform's stores replace other threads' ramps
       }
     } else if (PH != PH_ADJ && fwd && z < Z - 1) {
       if constexpr (TG) st_native(a.spec + (size_t)z * a.spec_step + (size_t)blockIdx.x * WW, v);
@@ -1007,44 +1021,35 @@ __global__ void __launch_bounds__(Geo<W>::T, Geo<W>::MINB) fused_multislice_kern
     } else if (PH != PH_FWD) {
       // probe-gradient spectrum with the shift adjoint, position gradient (objective.py:641-656)
       const float2* pf = a.probe_f + (size_t)p * WW;
-      FSum gy_c, gx_c;
-      // this element's spectrum times the conjugate ramp, and its share of the position gradient:
+      PSum gy_c, gx_c;
+      // this pack's spectrum times the conjugate ramp, and its share of the position gradient:
       // Re(smyx * conj(Pf) * F) with smyx = i*s*mask  ->  -(s*mask) * Im(conj(Pf) * F)
-      auto probe_element = [&](auto I, int ky, int kx, float2 ramp, float mk) {
-        constexpr int i = decltype(I)::value;
-        const float2 g = cmulc(wget(v, i), cscale(ramp, mk));
-        wset(v, i, g);
+      const float4* pf4 = reinterpret_cast<const float4*>(pf) + wo;
+      auto probe_pack = [&](int j, int ky, int kx, float2 rr, float2 ri, float2 mk) {
+        pcmul(v.re[j], v.im[j], rr, pneg(ri), ri);
         if (a.step_pos) {
-          const float im = cmulc(g, native_at(pf, i, t)).y;
-          gy_c += -(a.sy[ky] * mk) * im;
-          gx_c += -(a.sx[kx] * mk) * im;
+          const float4 f = pf4[j * 32];
+          const float2 im = pfma(v.im[j], make_float2(f.x, f.y), pneg(pmul(v.re[j], make_float2(f.z, f.w))));
+          gy_c.add(pmul(pmul(pdup(-a.sy[ky]), mk), im));
+          gx_c.add(pmul(pmul(make_float2(-a.sx[kx], -a.sx[kx + W / 2]), mk), im));
         }
       };
       if (a.probe_shift && a.mask_bin) {
         const uint32_t mbits = sbits[t];
-        if constexpr (PH == PH_WHOLE && kLean) {   // the first step's ramp, kept in shared memory
-          static_for<0, 32>([&](auto I) {
-            constexpr int i = decltype(I)::value;
-            probe_element(I, G::fky(t, i), G::fkx(t, i), sramp[i * T + t], ((mbits >> i) & 1u) ? 1.0f : 0.0f);
-          });
-        } else {
-          visit_sep_ramp<W>(a, t, dy, dx, [&](auto I, int ky, int kx, float2 ramp) {
-            probe_element(I, ky, kx, ramp, ((mbits >> decltype(I)::value) & 1u) ? 1.0f : 0.0f);
-          });
-        }
-      } else if (a.probe_shift) {
-        static_for<0, 32>([&](auto I) {
-          constexpr int i = decltype(I)::value;
-          const int ky = G::fky(t, i), kx = G::fkx(t, i);
-          const float mk = a.mask[ky * W + kx];
-          const float2 g = cmulc(wget(v, i), shift_ramp<W>(a, ky, kx, mk, dy, dx));
-          wset(v, i, g);
-          if (a.step_pos) {
-            const float im = cmulc(g, native_at(pf, i, t)).y;
-            gy_c += -(a.sy[ky] * mk) * im;
-            gx_c += -(a.sx[kx] * mk) * im;
-          }
+        visit_sep_ramp<W>(sph, t, [&](int j, int ky, int kx, float2 rr, float2 ri) {
+          const float2 mk = make_float2(((mbits >> (2 * j)) & 1u) ? 1.f : 0.f, ((mbits >> (2 * j + 1)) & 1u) ? 1.f : 0.f);
+          probe_pack(j, ky, kx, pmul(rr, mk), pmul(ri, mk), mk);
         });
+      } else if (a.probe_shift) {
+        __syncthreads();   // every warp has read its last operands from the exchange buffer
+        ramp_to_xbuf();
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+          const int ky = G::fky(t, 2 * j), kx = G::fkx(t, 2 * j);
+          const float2 r0 = xbuf[2 * j * T + t], r1 = xbuf[(2 * j + 1) * T + t];
+          probe_pack(j, ky, kx, make_float2(r0.x, r1.x), make_float2(r0.y, r1.y),
+                     make_float2(a.mask[ky * W + kx], a.mask[ky * W + kx + W / 2]));
+        }
       }
       if (a.step_probe) st_native(a.fprobe + ((size_t)b * a.Mp + p) * WW, v);
       if (a.step_pos) {

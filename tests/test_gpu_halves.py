@@ -11,8 +11,8 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("W,n,batches,opts", [
-    (64, 153, (153, 76), {}),                               # 306 and 152 blocks; one over what the GPU holds
-    (64, 160, (160, 80), dict(edge_mult=1.5, smooth_rolloff=0.08)),
+    (64, 229, (229, 114), {}),                              # 458 and 228 blocks; just over what the GPU holds
+    (64, 240, (240, 120), dict(edge_mult=1.5, smooth_rolloff=0.08)),
     (128, 58, (58, 57), {}),                                # 116 and 114 blocks: both sides of the line
     (128, 60, (60, 19), dict(step_pos=False, probe_shift=False, step_probe=False)),
     (128, 59, (59, 31), dict(step_obj=False, algorithm="ml")),
