@@ -300,7 +300,7 @@ __global__ void __launch_bounds__(512, 1) layered_fwd256_kernel(const float2* __
 // The kernel is compiled twice: PH = 1 runs the forward stages and the loss and leaves dL/dI
 // in dldi; PH = 2 starts from dldi and runs the adjoint stages. Each instance carries only
 // its own stages' code and live state (the one-kernel state machine spilled ~400 B per
-// thread; the two instances spill under 100 B). Propagation steps fold the forward cross
+// thread; the two instances spill 160 and 12 B). Propagation steps fold the forward cross
 // butterfly, the propagator and the inverse cross butterfly into one cluster exchange
 // (WinFFT256::cross_propagate).
 enum Stage256 : int { F_START = 0, F_SLICE, S_LOSS, A_START, A_RECOMP, A_SLICE, S_DONE };
@@ -492,8 +492,8 @@ __global__ void __launch_bounds__(512, 1) fused256_kernel(FusedArgs a) {
       const bool edge = a.use_edge && zstep == 0;
       const bool tab = !a.use_sep || edge;
       const float2* pr = a.prop_steps ? a.prop_steps + (size_t)zstep * (256 * 256) : (edge ? a.prop_edge : a.prop);
-      // separable: sum over q_y of P_y (sum over q_x of P_x Z_q), Z_q zero outside the band; a
-      // thread's packs share kx, so the x factors of the two column quadrants are held
+      // separable: P_y P_x of each quadrant, zero outside the band; a thread's packs share kx, so the
+      // x factors of the two column quadrants are held
       float2 xr[2], xi[2];
 #pragma unroll
       for (int qx = 0; qx < 2; ++qx) {
@@ -501,31 +501,20 @@ __global__ void __launch_bounds__(512, 1) fused256_kernel(FusedArgs a) {
         xr[qx] = make_float2(x[0].x, x[64].x);
         xi[qx] = adjoint ? make_float2(-x[0].y, -x[64].y) : make_float2(x[0].y, x[64].y);
       }
-      WinFFT256::cross_propagate(v, s.xbuf, cl, c, [&](int j, float2 (&zr)[4], float2 (&zi)[4], float2& re, float2& im) {
+      WinFFT256::cross_propagate(v, s.xbuf, cl, c, [&](int j, float2 (&zr)[4], float2 (&zi)[4]) {
         if (tab) {
-          WinFFT256::mul_quadrants(t, j, zr, zi, pr, adjoint, re, im);
+          WinFFT256::mul_quadrants(t, j, zr, zi, pr, adjoint);
           return;
         }
 #pragma unroll
-        for (int qy = 0; qy < 2; ++qy) {
-          float2 sr, si;
-#pragma unroll
-          for (int qx = 0; qx < 2; ++qx) {
-            const int q = 2 * qy + qx;
-            const uint32_t mb = sbits[q * T + t] >> (2 * j);
-            const float2 ar = make_float2((mb & 1u) ? zr[q].x : 0.f, (mb & 2u) ? zr[q].y : 0.f);
-            const float2 ai = make_float2((mb & 1u) ? zi[q].x : 0.f, (mb & 2u) ? zi[q].y : 0.f);
-            sr = qx ? pfma(ar, xr[qx], sr) : pmul(ar, xr[qx]);
-            si = qx ? pfma(ai, xr[qx], si) : pmul(ai, xr[qx]);
-            sr = pfma(ai, pneg(xi[qx]), sr);
-            si = pfma(ar, xi[qx], si);
-          }
-          const float4 y = spy[G::fky(2 * qy, t, 2 * j)];
-          const float2 yr = make_float2(y.x, y.y), yi = adjoint ? make_float2(-y.z, -y.w) : make_float2(y.z, y.w);
-          re = qy ? pfma(sr, yr, re) : pmul(sr, yr);
-          im = qy ? pfma(si, yr, im) : pmul(si, yr);
-          re = pfma(si, pneg(yi), re);
-          im = pfma(sr, yi, im);
+        for (int q = 0; q < 4; ++q) {
+          const uint32_t mb = sbits[q * T + t] >> (2 * j);
+          zr[q] = make_float2((mb & 1u) ? zr[q].x : 0.f, (mb & 2u) ? zr[q].y : 0.f);
+          zi[q] = make_float2((mb & 1u) ? zi[q].x : 0.f, (mb & 2u) ? zi[q].y : 0.f);
+          pcmul(zr[q], zi[q], xr[q & 1], xi[q & 1], pneg(xi[q & 1]));
+          const float4 y = spy[G::fky(q & 2, t, 2 * j)];
+          const float2 yi = adjoint ? make_float2(-y.z, -y.w) : make_float2(y.z, y.w);
+          pcmul(zr[q], zi[q], make_float2(y.x, y.y), yi, pneg(yi));
         }
       });
     } else {
