@@ -17,16 +17,16 @@ __device__ __forceinline__ void st_native128_conj(float2* base, const Win& v) {
   for (int j = 0; j < 16; ++j) p[j * 32] = pack4(v.re[j], pneg(v.im[j]));
 }
 
-// v *= w (conj_w: v *= conj(w)) for w in native order at base
-__device__ __forceinline__ void mul_native128(Win& v, const float2* base, bool conj_w) {
-  const float4* p = reinterpret_cast<const float4*>(base) + nword(0, threadIdx.x);
+// v *= the window that this thread's copies have brought to p (conj_w: its conjugate)
+__device__ __forceinline__ void mul_staged(Win& v, const float4* p, bool conj_w) {
+  cp_async_wait_all();
 #pragma unroll
   for (int j = 0; j < 16; ++j) {
     const float4 q = p[j * 32];
     const float2 wi = make_float2(q.z, q.w), ni = pneg(wi);
     pcmul(v.re[j], v.im[j], make_float2(q.x, q.y), conj_w ? ni : wi, conj_w ? wi : ni);
-    if ((j & 7) == 7) asm volatile("" ::: "memory");
   }
+  __syncwarp();   // the warp has read its part of the exchange buffer
 }
 
 // out = (accumulate ? out : 0) + a * v with a, out in native order
@@ -300,9 +300,11 @@ __global__ void __launch_bounds__(512, 1) layered_fwd256_kernel(const float2* __
 // The kernel is compiled twice: PH = 1 runs the forward stages and the loss and leaves dL/dI
 // in dldi; PH = 2 starts from dldi and runs the adjoint stages. Each instance carries only
 // its own stages' code and live state (the one-kernel state machine spilled ~400 B per
-// thread; the two instances spill 160 and 12 B). Propagation steps fold the forward cross
+// thread; the two instances spill 208 and 76 B). Propagation steps fold the forward cross
 // butterfly, the propagator and the inverse cross butterfly into one cluster exchange
-// (WinFFT256::cross_propagate).
+// (WinFFT256::cross_propagate). The next step's O_z comes by asynchronous copies into the warp's part
+// of the exchange buffer under the inverse transform's last round (plain loads: 81.2 -> 79.8 ms for 280
+// positions x 5 modes x 24 slices, 3.16 -> 3.06 ms for 28 x 2 x 12).
 enum Stage256 : int { F_START = 0, F_SLICE, S_LOSS, A_START, A_RECOMP, A_SLICE, S_DONE };
 
 template <int PH>
@@ -353,6 +355,7 @@ __global__ void __launch_bounds__(512, 1) fused256_kernel(FusedArgs a) {
   }
   __syncthreads();
 
+  float4* xw = reinterpret_cast<float4*>(s.xbuf + (t >> 5) * WinFFT<128>::WPART) + (t & 31);   // this thread's O_z
   Win v;
   while (stage != S_DONE) {
     const bool fwd_stage = FWD;
@@ -433,7 +436,7 @@ __global__ void __launch_bounds__(512, 1) fused256_kernel(FusedArgs a) {
       do_inv = true;
     } else if (FWD) {   // F_SLICE
       if (store_stack && z % K == 0) st_native128_conj(wpart(a.stack, stack_win(z, p, m)), v);
-      mul_native128(v, part(a.obl, ((size_t)b * Z + z) * Mo + m), false);
+      mul_staged(v, xw, false);
       do_fwd = true;
       do_inv = z < Z - 1;
     } else if (stage == A_RECOMP) {
@@ -445,7 +448,7 @@ __global__ void __launch_bounds__(512, 1) fused256_kernel(FusedArgs a) {
       }
       st_native128_conj(wpart(a.seg, (size_t)b * K + (z - z0)), v);
       if (z < zl) {
-        mul_native128(v, part(a.obl, ((size_t)b * Z + z) * Mo + m), false);
+        mul_staged(v, xw, false);
         do_fwd = true;
         do_inv = true;
       } else {
@@ -457,7 +460,7 @@ __global__ void __launch_bounds__(512, 1) fused256_kernel(FusedArgs a) {
         const float2* src = K == 1 ? part(a.stack, stack_win(z, p, m)) : part(a.seg, (size_t)b * K + (z - z0));
         madd_native128(wpart(a.gsum, ((size_t)b * Z + z) * Mo + m), src, v, p > 0);
       }
-      mul_native128(v, part(a.obl, ((size_t)b * Z + z) * Mo + m), true);
+      mul_staged(v, xw, true);
       if (z > 0) {
         do_fwd = true;
         do_inv = true;
@@ -544,11 +547,6 @@ __global__ void __launch_bounds__(512, 1) fused256_kernel(FusedArgs a) {
       }
       if (do_inv) WinFFT256::cross(v, s.xbuf, cl, c);
     }
-    if (do_inv) {
-      WinFFT256::twiddle(v, s.tw256, c, true);
-      WinFFT<128>::inverse(v, s.xbuf, s.tw1, s.tw2);
-    }
-
     // ------------------------------------------------ next step
     if (FWD) {
       if (stage == F_START) {
@@ -587,6 +585,22 @@ __global__ void __launch_bounds__(512, 1) fused256_kernel(FusedArgs a) {
         stage = S_DONE;
       }
     }
+
+    // ------------------------------------------------ inverse transform, the next step's O_z copied into
+    // the warp's part of the exchange buffer behind its register-only last round
+    if (do_inv) {
+      WinFFT256::twiddle(v, s.tw256, c, true);
+      WinFFT<128>::inverse_head(v, s.xbuf, s.tw1, s.tw2);
+      __syncwarp();
+    }
+    if (FWD ? stage == F_SLICE : stage == A_SLICE || (stage == A_RECOMP && z < zl)) {
+      const int mn = FWD ? k / Mp : k % Mo;
+      const float4* o = reinterpret_cast<const float4*>(part(a.obl, ((size_t)b * Z + z) * Mo + mn)) + nword(0, t);
+#pragma unroll
+      for (int j = 0; j < 16; ++j) cp_async16(xw + j * 32, o + j * 32);
+      cp_async_commit();
+    }
+    if (do_inv) WinFFT<128>::inverse_tail(v);
   }
 }
 
