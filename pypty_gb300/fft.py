@@ -19,9 +19,11 @@ def _run(arr, axes, inverse, shift):
     eng = default_engine()
     t = t.to(device=eng.device, dtype=torch.complex64)
     a0, a1 = (ax % t.dim() for ax in axes)
-    moved = torch.movedim(t, (a0, a1), (-2, -1)).contiguous()
-    out = eng.fft2(moved, inverse=inverse, shift=shift)
-    out = torch.movedim(out, (-2, -1), (a0, a1))
+    in_place = (a0, a1) == (t.dim() - 2, t.dim() - 1)   # the axes are the last two already
+    moved = t if in_place else torch.movedim(t, (a0, a1), (-2, -1))
+    out = eng.fft2(moved.contiguous(), inverse=inverse, shift=shift)
+    if not in_place:
+        out = torch.movedim(out, (-2, -1), (a0, a1))
     if is_numpy:
         res = out.cpu().numpy()
         return res.astype(np.complex128) if in_dtype in (torch.complex128, torch.float64) else res

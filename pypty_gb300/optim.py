@@ -25,6 +25,7 @@ charge flipping, Gaussian filters, object resizing and position puzzling.
 from __future__ import annotations
 
 import ctypes
+import math
 import sys
 from dataclasses import dataclass, field
 
@@ -58,7 +59,7 @@ def fourier_clean_(x: torch.Tensor, cutoff=None, rolloff=0.0, mask=None, out: to
     if x.dim() < 2:
         raise ValueError("fourier_clean_ needs at least 2 axes")
     ny, nx = int(x.shape[0]), int(x.shape[1])
-    k = int(np.prod(x.shape[2:])) if x.dim() > 2 else 1
+    k = math.prod(x.shape[2:])
     if out is None:
         out = torch.empty_like(x)
     if dx is not None and (dx.shape != x.shape or dx.dtype != x.dtype or not dx.is_contiguous()):
@@ -73,6 +74,12 @@ def fourier_clean_(x: torch.Tensor, cutoff=None, rolloff=0.0, mask=None, out: to
 def _clean_tables(eng: Engine, ny, nx, cutoff, rolloff, mask):
     """Twiddle and band-limit tables of one (ny, nx, cutoff, rolloff), prepared once per
     engine (``pty_fourier_clean_prepare``); a caller-given mask is prepared every call."""
+    if mask is None:
+        c32, r32 = np.float32(cutoff), np.float32(rolloff)
+        key = "fourier_clean:%d:%d:%08x:%08x" % (ny, nx, c32.view(np.uint32), r32.view(np.uint32))
+        ws = eng._aux.get(key)
+        if ws is not None:
+            return ws
     n = ctypes.c_size_t(0)
     _lib.check(_lib.lib().pty_fourier_clean_workspace_bytes(ny, nx, ctypes.byref(n)),
                "pty_fourier_clean_workspace_bytes (object extents must be powers of two in [64, 8192])")
@@ -85,13 +92,9 @@ def _clean_tables(eng: Engine, ny, nx, cutoff, rolloff, mask):
         _lib.check(_lib.lib().pty_fourier_clean_prepare(ny, nx, 0.0, 0.0, m.data_ptr(), ws.data_ptr(), ws.numel(),
                                                         _stream(eng)), "pty_fourier_clean_prepare")
         return ws
-    c32, r32 = np.float32(cutoff), np.float32(rolloff)
-    key = "fourier_clean:%d:%d:%08x:%08x" % (ny, nx, c32.view(np.uint32), r32.view(np.uint32))
-    ws = eng._aux.get(key)
-    if ws is None:
-        ws = eng.aux(key, int(n.value))
-        _lib.check(_lib.lib().pty_fourier_clean_prepare(ny, nx, float(c32), float(r32), None, ws.data_ptr(),
-                                                        ws.numel(), _stream(eng)), "pty_fourier_clean_prepare")
+    ws = eng.aux(key, int(n.value))
+    _lib.check(_lib.lib().pty_fourier_clean_prepare(ny, nx, float(c32), float(r32), None, ws.data_ptr(),
+                                                    ws.numel(), _stream(eng)), "pty_fourier_clean_prepare")
     return ws
 
 

@@ -56,3 +56,23 @@ def test_band_limit_runs(Mp, nx):
         assert np.array_equal(s0, s1) and np.array_equal(g0, g1)
         assert np.abs(l0 - l1).max() <= 1e-12 * np.abs(l1).max()
         assert rel_l2(o0, o1) <= 2e-6 and rel_l2(p0, p1) <= 2e-6
+
+
+@pytest.mark.parametrize("axes,order", [((1, 2), (0, 1, 2)), ((-2, -1), (2, 1, 0)), ((0, 1), (1, 2, 0)), ((2, 1), (0, 2, 1)),
+                                        ((2, 0), (2, 0, 1))])
+def test_fft_wrapper_axes(axes, order):
+    """The wrapper's axes, last two or not, of contiguous and permuted tensors against NumPy."""
+    import torch
+    from pypty_gb300 import fft
+    rng = np.random.default_rng(3)
+    shape = [64, 64, 64]
+    other = ({0, 1, 2} - {a % 3 for a in axes}).pop()
+    shape[other] = 3
+    mem = [shape[i] for i in order]                     # the tensor's axis order in memory
+    a = (rng.normal(size=mem) + 1j * rng.normal(size=mem)).astype(np.complex64).transpose(np.argsort(order))
+    t = torch.from_numpy(np.ascontiguousarray(a.transpose(order))).cuda().permute(*np.argsort(order).tolist())
+    assert tuple(t.shape) == tuple(shape)
+    for f, g in ((fft.fft2, np.fft.fft2), (fft.ifft2, np.fft.ifft2)):
+        got = f(t, axes=axes)
+        assert got.is_contiguous()
+        assert rel_l2(got.cpu().numpy(), g(a.astype(np.complex128), axes=axes)) <= 1e-6
