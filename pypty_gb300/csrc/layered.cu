@@ -14,7 +14,7 @@
 // probe-gradient chunk sums and the FP64 loss / position-gradient reductions are the fused
 // path's deterministic kernels. Per batch of positions (pypty/objective.py:425-705):
 //   gather + band-limit object windows; probe spectrum x ramp -> probe per position;
-//   Z slices: stack conj(psi), psi *= O_z, psi = IDFT(DFT(psi) P);  far field, loss, dL/dPsi;
+//   Z slices: stack conj(psi) (fused route: psi), psi *= O_z, psi = IDFT(DFT(psi) P);  far field, loss, dL/dPsi;
 //   Z slices back: dO_z = sum_p stack * g, g *= conj(O_z), g = IDFT(DFT(g) conj P);
 //   band-limit and scatter dO; probe-gradient spectra (shift adjoint, position gradient).
 #include <cuda_runtime.h>
