@@ -442,10 +442,13 @@ __device__ __forceinline__ float sqrt_heron(float x, float& r) {
   return (x == 0.0f || x == INFINITY) ? x : t;
 }
 
-// a / b from r, about 1/b: the quotient with its remainder put back (no slow-path branch either)
+// a / b from r, about 1/b: the quotient with its remainder put back (Markstein's correction, IBM J. Res.
+// Dev. 34, 1990; no slow-path branch either). Where a or b is infinite, or a / b is, there is no remainder
+// (inf - inf, 0 * inf) and a r is the quotient.
 __device__ __forceinline__ float quotient(float a, float b, float r) {
   const float q = a * r;
-  return fmaf(fmaf(-q, b, a), r, q);
+  const float e = fmaf(fmaf(-q, b, a), r, q);
+  return e == e ? e : q;
 }
 
 // dL/dI of one detector pixel for the loss `alg` (pypty/objective.py:527-559), with the
