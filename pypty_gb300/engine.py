@@ -94,6 +94,7 @@ class Engine:
         self._ws = None
         self._aux = {}
         self._aux_events = {}
+        self._clean_tables = {}     # optim._clean_tables
         # two page-locked geometry buffers used in turn, each with the event of the call that
         # last read it: the host fills one while the GPU may still run the previous call
         self._stages = [None, None]
@@ -107,7 +108,7 @@ class Engine:
             self._ws = torch.empty(max(nbytes, 256), dtype=torch.uint8, device=self.device)
         return self._ws
 
-    def aux(self, key: str, nbytes: int) -> torch.Tensor:
+    def aux(self, key, nbytes: int) -> torch.Tensor:
         """A device buffer of at least nbytes kept per key (small tables, optimizer state),
         separate from the loss-and-gradient workspace."""
         buf = self._aux.get(key)

@@ -73,28 +73,46 @@ def fourier_clean_(x: torch.Tensor, cutoff=None, rolloff=0.0, mask=None, out: to
 
 def _clean_tables(eng: Engine, ny, nx, cutoff, rolloff, mask):
     """Twiddle and band-limit tables of one (ny, nx, cutoff, rolloff), prepared once per
-    engine (``pty_fourier_clean_prepare``); a caller-given mask is prepared every call."""
+    engine (``pty_fourier_clean_prepare``) and kept for calls on any stream: the first call on
+    another stream than the one that prepared them waits for that. A caller-given mask is
+    prepared by every call, into a buffer of its stream's. Tables prepared while the stream is
+    being captured exist only when the graph runs: they belong to the captured call."""
+    stream = torch.cuda.current_stream(eng.device)
+    st = stream.cuda_stream
+    key = None
     if mask is None:
         c32, r32 = np.float32(cutoff), np.float32(rolloff)
-        key = "fourier_clean:%d:%d:%08x:%08x" % (ny, nx, c32.view(np.uint32), r32.view(np.uint32))
-        ws = eng._aux.get(key)
-        if ws is not None:
+        key = (ny, nx, c32.tobytes(), r32.tobytes())
+        kept = eng._clean_tables.get(key)
+        if kept is not None:
+            ws, ready, ordered = kept
+            # a stream under capture runs nothing now, and may not wait for an event of before
+            if st not in ordered and not torch.cuda.is_current_stream_capturing():
+                stream.wait_event(ready)
+                ws.record_stream(stream)
+                ordered.add(st)
             return ws
     n = ctypes.c_size_t(0)
     _lib.check(_lib.lib().pty_fourier_clean_workspace_bytes(ny, nx, ctypes.byref(n)),
                "pty_fourier_clean_workspace_bytes (object extents must be powers of two in [64, 8192])")
+    m = None
+    if key is not None or torch.cuda.is_current_stream_capturing():
+        ws = torch.empty(int(n.value), dtype=torch.uint8, device=eng.device)
+    else:
+        ws = eng.aux(("fourier_clean_given_mask", st), int(n.value))
     if mask is not None:
         m = mask if isinstance(mask, torch.Tensor) else torch.from_numpy(np.ascontiguousarray(
             np.asarray(mask.get() if hasattr(mask, "get") else mask, dtype=np.float32)))
-        m = m.to(device=eng.device, dtype=torch.float32).reshape(ny, nx).contiguous()
-        ws = eng.aux("fourier_clean_given_mask", int(n.value))
-        eng._aux["fourier_clean_mask_src"] = m     # alive until the kernels have read it
-        _lib.check(_lib.lib().pty_fourier_clean_prepare(ny, nx, 0.0, 0.0, m.data_ptr(), ws.data_ptr(), ws.numel(),
-                                                        _stream(eng)), "pty_fourier_clean_prepare")
-        return ws
-    ws = eng.aux(key, int(n.value))
-    _lib.check(_lib.lib().pty_fourier_clean_prepare(ny, nx, float(c32), float(r32), None, ws.data_ptr(),
-                                                    ws.numel(), _stream(eng)), "pty_fourier_clean_prepare")
+        if m.dtype != torch.float32 or m.device != ws.device or m.shape != (ny, nx) or not m.is_contiguous():
+            m = m.to(device=eng.device, dtype=torch.float32).reshape(ny, nx).contiguous()
+        eng._aux["fourier_clean_mask_src", st] = m     # alive until the kernels have read it
+        c32 = r32 = 0.0
+    _lib.check(_lib.lib().pty_fourier_clean_prepare(ny, nx, float(c32), float(r32), None if m is None else m.data_ptr(),
+                                                    ws.data_ptr(), ws.numel(), st), "pty_fourier_clean_prepare")
+    if key is not None and not torch.cuda.is_current_stream_capturing():
+        ready = torch.cuda.Event()
+        ready.record(stream)
+        eng._clean_tables[key] = (ws, ready, {st})
     return ws
 
 
