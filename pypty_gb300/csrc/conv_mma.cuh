@@ -205,8 +205,7 @@ __global__ void __launch_bounds__(ConvCfg::THREADS, 2)
       umma::mma_commit(&bar);
     }
   }
-  mbar_wait(&bar, par, &err);
-  umma::fence_after_sync();
+  umma::wait_mma(&bar, par, &err);
   const bool slow = __syncthreads_or(bad || err);   // also: every MMA has read the tile
   bf16* so = reinterpret_cast<bf16*>(sm);           // [32 channels][16][16]
   {
@@ -320,7 +319,8 @@ __global__ void __launch_bounds__(WgradCfg::THREADS, 2)
   for (uint32_t e = chunks * C::D_CHUNK / 16 + tid; e < C::D_BYTES / 16; e += C::THREADS)
     reinterpret_cast<uint4*>(sd)[e] = make_uint4(0u, 0u, 0u, 0u);
   const long long b0 = blk * per, b1 = b0 + per < total ? b0 + per : total;
-  for (long long b = b0; b < b1; ++b) {
+  bool failed = false;   // a wait ran out in some thread: the whole share becomes NaN
+  for (long long b = b0; b < b1 && !failed; ++b) {
     const int n = (int)(b / tiles), tile = (int)(b % tiles);
     const int y0 = (tile / tiles_x) * C::TH, x0 = (tile % tiles_x) * C::TW;
     // dy: 16 chunks of 8 channels x 256 pixels, a task is 8 channels x 2 pixels
@@ -362,7 +362,7 @@ __global__ void __launch_bounds__(WgradCfg::THREADS, 2)
 #pragma unroll
       for (int k = 0; k < 8; ++k) bs[k] += t[k];
     }
-    for (int g = 0; g < C::TH / C::GROUP; ++g) {
+    for (int g = 0; g < C::TH / C::GROUP && !failed; ++g) {
       if (tid == 0) {
         umma::fence_after_sync();
         constexpr uint32_t idesc = umma::idesc_bf16_f32(128, C::N) | (1u << 15) | (1u << 16);   // A, B MN-major
@@ -378,8 +378,7 @@ __global__ void __launch_bounds__(WgradCfg::THREADS, 2)
         }
         umma::mma_commit(&bar);
       }
-      mbar_wait(&bar, par, &err);
-      umma::fence_after_sync();
+      umma::wait_mma(&bar, par, &err);
       const uint32_t t0 = tmem + ((uint32_t)(32 * q) << 16) + share * C::SHARE;
       static_assert(C::SHARE == 72, "32 + 32 + 8 columns");
       float v[32], u[8];
@@ -393,9 +392,14 @@ __global__ void __launch_bounds__(WgradCfg::THREADS, 2)
 #pragma unroll
       for (int k = 0; k < 8; ++k) acc[64 + k] += u[k];
       umma::fence_before_sync();
-      __syncthreads();   // the accumulators are read (and, after the last group, the tile is)
+      // the accumulators are read (and, after the last group, the tile is)
+      failed = __syncthreads_or(err);
       umma::fence_after_sync();
     }
+  }
+  if (failed) {   // once more, bounded, before TMEM goes
+    uint32_t last = par ^ 1u;
+    mbar_wait(&bar, last, nullptr);
   }
   umma::fence_before_sync();
   __syncthreads();
@@ -406,7 +410,7 @@ __global__ void __launch_bounds__(WgradCfg::THREADS, 2)
 #pragma unroll
     for (int k = 0; k < C::SHARE; ++k) {
       const int col = share * C::SHARE + k, tap = col / C::CI, i = i0 + col % C::CI;
-      if (i < Ci) pw[((size_t)tap * Ci + i) * Co + o] = err ? NAN : acc[k];
+      if (i < Ci) pw[((size_t)tap * Ci + i) * Co + o] = failed ? NAN : acc[k];
     }
   }
   if (i0 == 0) {
@@ -415,7 +419,7 @@ __global__ void __launch_bounds__(WgradCfg::THREADS, 2)
     for (int k = 0; k < 8; ++k) {
 #pragma unroll
       for (int s = 8; s > 0; s >>= 1) bs[k] += __shfl_down_sync(0xffffffffu, bs[k], s, 16);
-      if ((tid & 15) == 0 && o0 + 8 * ch + k < Co) pbias[(size_t)blk * Co + o0 + 8 * ch + k] = bs[k];
+      if ((tid & 15) == 0 && o0 + 8 * ch + k < Co) pbias[(size_t)blk * Co + o0 + 8 * ch + k] = failed ? NAN : bs[k];
     }
   }
 }

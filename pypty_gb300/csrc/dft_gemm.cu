@@ -171,8 +171,7 @@ __global__ void __launch_bounds__(THREADS, 1)
   auto drain = [&](int kc) {
     const int buf = kc & 1;
     drained = kc;
-    mbar_wait(&drain_bar[buf], drain_par[buf], &e);
-    umma::fence_after_sync();
+    umma::wait_mma(&drain_bar[buf], drain_par[buf], &e);
     // exact variant: this thread's row (TMEM lane 32 q + lane) carries scale 2^(E - 7) from A and
     // 2^-7 from B
     float rs = 1.0f;

@@ -62,18 +62,31 @@ __device__ __forceinline__ void mma_commit(uint64_t* bar) {
 __device__ __forceinline__ void fence_before_sync() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_after_sync() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
+// The .aligned instructions below want the warp's lanes together. Lanes that took a branch of their own
+// (the thread that issues) or left a waiting loop at different trips are brought together first: here for
+// allocation and release, in wait_mma for the loads.
+
+// every lane: wait (bounded) for the MMAs committed to `bar`, ready to load from TMEM
+__device__ __forceinline__ void wait_mma(uint64_t* bar, uint32_t& parity, int* err) {
+  mbar_wait(bar, parity, err);
+  __syncwarp();
+  fence_after_sync();
+}
+
 // warp-wide: allocate ncols TMEM columns (power of two >= 32); the address lands in *dst
 __device__ __forceinline__ void tmem_alloc(uint32_t* dst, uint32_t ncols) {
+  __syncwarp();
   asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(dst)), "r"(ncols)
                : "memory");
   asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
 }
 
 __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
+  __syncwarp();
   asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
 
-// warp-wide: lane l of the warp receives columns [col, col + 32) of TMEM lane (lane_base + l)
+// warp-wide, after wait_mma: lane l of the warp receives columns [col, col + 32) of TMEM lane (lane_base + l)
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
   uint32_t r[32];
   asm volatile(
