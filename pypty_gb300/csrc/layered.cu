@@ -1120,7 +1120,8 @@ inline LPlan make_lplan(const pty_problem_t* p, int engine, const pty_variant_t*
     q.o_pprop_edge = take(q.pos_prop && edge ? (size_t)q.Bb * WWs * c8 : 0);
     q.fused = engine == PTY_DFT_FP32_FFT && q.W <= 128 && !(q.pos_prop && q.per_step);
   }
-  q.o_dob = take((q.fused ? q.Mp : 1) * nobw * WWs * c8);   // one contribution window per probe mode
+  // gradient windows: the fused halves leave one contribution per probe mode in the place of its wave
+  q.o_dob = q.fused ? q.o_stack : take(nobw * WWs * c8);
   q.o_tmp = take((q.fused ? 0 : nobw) * WWs * c8);
   q.o_tilt_part = take(q.fused && q.inside_grad ? nwave * 2 * sizeof(double) : 0);
   q.o_tilt_w = take(q.fused && q.inside_grad ? (size_t)q.Z * sizeof(float) : 0);
@@ -1565,7 +1566,6 @@ struct Run {
         vb.tw = fp32_twiddles();
         vb.obl = ob;
         vb.stack = stack;
-        vb.gsum = dob;
         vb.pnat = pbs;     // free between the incoming probe's transform and the probe gradient
         vb.wnat = psi2;    // free outside the far field
         vb.fprobe = pb;    // the incoming probe is no longer needed in the adjoint

@@ -535,8 +535,8 @@ FusedArgs var_args(const VarBatch& a) {
   fa.corr = reinterpret_cast<const float*>(a.pos);   // read and not used
   fa.seq = a.seq;
   fa.tw = a.tw;
-  fa.stack = a.stack;
-  fa.gsum = a.gsum;
+  fa.stack = fa.gsum = a.stack;
+  fa.stack_obj_first = 1;
   fa.fprobe = a.fprobe;
   fa.spec = a.spec;
   fa.spec_step = (size_t)a.Bn * a.Mp * a.Mo * W * W;
@@ -598,7 +598,7 @@ int var_adjoint(const VarBatch& a, const float2* g, bool step_obj, float2* probe
     return rc;
   if (step_obj) {
     prof_mark(st, KID_GRAD_WINDOWS);
-    if ((rc = launch_grad_windows<W>(a.gsum, a.mask_sc, a.tw, a.Mp, a.Bn * a.Z * a.Mo, st))) return rc;
+    if ((rc = launch_grad_windows<W>(a.stack, a.mask_sc, a.tw, a.Mp, a.Bn * a.Z * a.Mo, st))) return rc;
   }
   if (probe_grad) {
     prof_mark(st, KID_LAYOUT);

@@ -263,8 +263,8 @@ struct VarBatch {
   const float2 *obj;                    // slice-major object
   const float2 *prop, *prop_edge, *prop_steps, *prop_pos, *prop_pos_edge;   // scaled by 1/W^2
   const float *mask, *mask_sc, *sx;
-  float2 *tw, *obl, *stack, *gsum, *pnat, *wnat;   // workspace: twiddles, object windows, waves, gradient
-                                        // contributions, probes and waves in native order
+  float2 *tw, *obl, *stack, *pnat, *wnat;   // workspace: twiddles, object windows, the waves (whose places
+                                        // the gradient contributions take), probes and waves in native order
   float2* fprobe;                       // native probe gradient [Bn*Mp]
   float2* spec;                         // inside-tilt gradient: step spectra, or nullptr
   const float* tilt_w;                  // step weights, or nullptr
@@ -276,7 +276,7 @@ struct VarBatch {
 template <int W>
 int var_forward(const VarBatch& a, const float2* probes, bool shared, float2* exit, cudaStream_t st);
 // dL/d(exit wave) (natural) -> gradient windows (natural, window (b, k) at ((b*Z*Mo + k)*Mp) * W^2 of
-// gsum, when step_obj) and the probe gradient summed over object modes (natural [Bn*Mp], when given)
+// stack, when step_obj) and the probe gradient summed over object modes (natural [Bn*Mp], when given)
 template <int W>
 int var_adjoint(const VarBatch& a, const float2* g, bool step_obj, float2* probe_grad, cudaStream_t st);
 

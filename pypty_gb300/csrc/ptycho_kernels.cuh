@@ -347,7 +347,8 @@ struct FusedArgs {
   const int* seq;           // batch's sequence entries
   const float* measured;    // (N, W, W) detector (fftshifted) order
   const float2* tw;
-  float2* stack;            // input waves (256 windows: their conjugates), native real [Bb*Z*Mp*Mo]
+  float2* stack;            // input waves (256 windows: their conjugates), native real [Bb*Z*Mp*Mo], or
+  int stack_obj_first;      // [Bb*Z*Mo*Mp] with stack_obj_first: gsum may then be the stack itself
   float2* gsum;             // object-gradient contributions, native real [Bb*Z*Mo*Mp] (probe mode innermost)
   float2* fprobe;           // FFT of the per-position probe gradient, native freq [Bb*Mp]
   const float2* gbuf;       // adjoint half: a given dL/d(exit wave), native real [Bb*Mp*Mo], and a
@@ -629,7 +630,8 @@ __global__ void __launch_bounds__(Geo<W>::T, Geo<W>::MINB) fused_multislice_kern
   uint32_t ph_x = 0, ph_side = 0;
 
   auto obl_ptr = [&](int z) { return a.obl + (((size_t)b * Z + z) * a.Mo + m) * WW; };
-  auto stack_ptr = [&](int z) { return a.stack + ((((size_t)b * Z + z) * a.Mp + p) * a.Mo + m) * WW; };
+  const int smode = PH != PH_WHOLE && a.stack_obj_first ? m * a.Mp + p : p * a.Mo + m;
+  auto stack_ptr = [&](int z) { return a.stack + (((size_t)b * Z + z) * nmodes + smode) * WW; };
   // O_z of step s >= 1: the adjoint steps read it from the exchange buffer, the forward steps
   // through the side buffer
   auto xsrc = [&](int s) -> const float2* { return obl_ptr(s <= Z ? s - 1 : 2 * Z - s); };
@@ -776,7 +778,8 @@ __global__ void __launch_bounds__(Geo<W>::T, Geo<W>::MINB) fused_multislice_kern
         // buffer ([position][slice][object mode][probe mode]); grad_windows_kernel adds the
         // probe modes in ascending order before the band limit (multislice_core.py:184-191), so
         // the adjoint needs no cluster barrier and no remote reads. Elements < NST replace
-        // psi_z in the side buffer, whence a bulk copy takes them out behind the transform.
+        // psi_z in the side buffer, whence a bulk copy takes them out behind the transform. The
+        // window may be psi_z's own: it is read by this warp alone, and has been when it is written.
         float4* g4 = reinterpret_cast<float4*>(contrib_ptr(z));
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
