@@ -136,13 +136,17 @@ inline Plan make_plan(const pty_problem_t* p, bool split = false) {
   // form the loss once per position, for two more launches (~10 us of a call). Whole pass against
   // halves: 128 px, 768 blocks x 20 slices, four batches, 18.4 -> 16.4 ms; 128 blocks x 7 slices,
   // three batches, 1036 -> 1004 us; 108 blocks x 3 slices 248 -> 251 us; 64 px, 1200 blocks x 8
-  // slices 802 -> 727 us, 480 x 6 365 -> 349 us, 440 x 6 278 -> 283 us, 400 x 1 98 -> 110 us.
+  // slices 802 -> 727 us, 480 x 6 365 -> 349 us, 440 x 6 278 -> 283 us, 400 x 1 98 -> 110 us. The line does
+  // not look at the number of slices: just above it calls of one slice would still be faster whole (620 x 1
+  // 137 us against 156, 128 px 152 x 1 130 against 149; 760 x 4 349 against 343, 152 x 3 345 against 337).
   const int blocks = q.Bb * q.Mp;
   q.halves = !w256 && !split && q.Mo == 1 && q.Mp > 1 && blocks > (q.W == 64 ? resident_blocks(64) : kSMs * 3 / 4);
   const bool far = w256 || split || q.halves;
-  q.s_psi = align_up(far ? (size_t)q.Bb * q.Mp * q.Mo * WW * c8 : 0);
+  // The halves' far-field waves lie where their probe-gradient spectra go: a block has read its wave before
+  // it writes its spectrum. (The split calls keep theirs: pty_backward may run again on one workspace.)
+  q.s_psi = q.halves ? q.s_fprobe : align_up(far ? (size_t)q.Bb * q.Mp * q.Mo * WW * c8 : 0);
   q.s_dldi = align_up(far ? (size_t)q.Bb * WW * f4 : 0);
-  q.o_psi = take(q.nbuf * q.s_psi);
+  q.o_psi = q.halves ? q.o_fprobe : take(q.nbuf * q.s_psi);
   q.o_dldi = take(q.nbuf * q.s_dldi);
   q.o_pgr = take(w256 && q.Mo > 1 ? (size_t)q.Bb * q.Mp * WW * c8 : 0);
   q.o_seg = take(q.ckpt > 1 ? (size_t)q.Bb * q.ckpt * WW * c8 : 0);
