@@ -139,9 +139,10 @@ __device__ __forceinline__ void transform(float2 (&v)[EPT], float2* sm, const Sr
 }
 
 // MODE 0: pass X (forward, optional a + step b); 1: pass Y (forward, mask, inverse);
-// 2: pass X' (inverse, scaled).
+// 2: pass X' (inverse, scaled). Lines of 2048 to 8192 points; shorter ones are clean_line_kernel's.
 template <int N, int MODE>
 __global__ void __launch_bounds__(TPB, MODE == 1 ? 1 : 2) clean_pass_kernel(PassArgs A) {
+  static_assert(N >= 2048, "shorter lines run in clean_line_kernel");
   extern __shared__ float2 sm[];
   constexpr int KB = TILE / N;
   const int s = threadIdx.x % KB;

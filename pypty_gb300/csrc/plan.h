@@ -20,7 +20,7 @@ struct Plan {
   int W, Ny, Nx, Z, Mo, Mp, N, nseq, Bb, nbatch, zm, ntx, nty, ntiles, nchunk, chunk;
   size_t o_tw, o_mask, o_mask_sc, o_prop, o_prop_edge, o_pyx, o_sx, o_sy, o_probe_f;
   size_t o_pos, o_corr, o_seq, o_obj, o_grad, o_obl, o_stack, o_gsum, o_fprobe, o_partial;
-  size_t o_lists, o_counts, o_loss_part, o_pos_part, o_sim, o_err, o_psi, o_dldi, o_pgr, o_seg, o_gpark;
+  size_t o_lists, o_counts, o_loss_part, o_pos_part, o_err, o_psi, o_dldi, o_pgr, o_seg, o_gpark;
   size_t total;
   int ckpt;   // kept slices every ckpt (256 windows)
   bool split;   // one batch with every position: pty_forward / pty_backward
@@ -128,7 +128,6 @@ inline Plan make_plan(const pty_problem_t* p, bool split = false) {
   q.o_counts = take((size_t)q.ntiles * sizeof(int));
   q.o_loss_part = take((size_t)q.nseq * 2 * sizeof(double));
   q.o_pos_part = take((size_t)q.nseq * q.Mp * 2 * sizeof(double));
-  q.o_sim = take((size_t)q.Bb * WW * f4);
   q.o_err = take(sizeof(int));
   const bool w256 = q.W == 256;
   // The whole pass of 64- and 128-px windows runs as its halves (see FusedPart) when a batch has
@@ -145,9 +144,9 @@ inline Plan make_plan(const pty_problem_t* p, bool split = false) {
   // The halves' far-field waves lie where their probe-gradient spectra go: a block has read its wave before
   // it writes its spectrum. (The split calls keep theirs: pty_backward may run again on one workspace.)
   q.s_psi = q.halves ? q.s_fprobe : align_up(far ? (size_t)q.Bb * q.Mp * q.Mo * WW * c8 : 0);
-  q.s_dldi = align_up(far ? (size_t)q.Bb * WW * f4 : 0);
+  q.s_dldi = align_up((size_t)q.Bb * WW * f4);   // read and written where `far` holds
   q.o_psi = q.halves ? q.o_fprobe : take(q.nbuf * q.s_psi);
-  q.o_dldi = take(q.nbuf * q.s_dldi);
+  q.o_dldi = take((far ? q.nbuf : 1) * q.s_dldi);
   q.o_pgr = take(w256 && q.Mo > 1 ? (size_t)q.Bb * q.Mp * WW * c8 : 0);
   q.o_seg = take(q.ckpt > 1 ? (size_t)q.Bb * q.ckpt * WW * c8 : 0);
   q.o_gpark = take(q.ckpt > 1 ? (size_t)q.Bb * WW * c8 : 0);
@@ -193,7 +192,7 @@ int set_smem(K kernel, size_t bytes) {
 struct MsPlan {
   int W, B, Z, Mp, Mo, Ny, Nx, zm, ntx, nty, ntiles;
   size_t o_tw, o_prop, o_prop_edge, o_mask, o_mask_sc, o_pyx, o_probe_b, o_obl, o_stack, o_gbuf, o_gsum;
-  size_t o_fprobe, o_grad, o_lists, o_counts, o_pos, o_seq, o_corr, o_err, o_parts, total;
+  size_t o_fprobe, o_grad, o_lists, o_counts, o_pos, o_seq, o_corr, o_err, total;
 };
 
 inline MsPlan make_ms_plan(int W, int B, int Z, int Mp, int Mo, int Ny, int Nx) {
@@ -231,7 +230,6 @@ inline MsPlan make_ms_plan(int W, int B, int Z, int Mp, int Mo, int Ny, int Nx) 
   q.o_seq = take((size_t)B * sizeof(int));
   q.o_corr = take((size_t)B * 2 * sizeof(float));
   q.o_err = take(sizeof(int));
-  q.o_parts = take((size_t)B * (2 + 2 * Mp) * sizeof(double));
   q.total = o;
   return q;
 }
