@@ -194,8 +194,7 @@ __global__ void __launch_bounds__(TPB, MODE == 1 ? 1 : 2) clean_pass_kernel(Pass
 // shared memory under the loads of the lines. Bound by the latency of load, transform and store with
 // 16 warps on an SM (32 points a thread are 128 registers) and by a last wave that is nearly empty;
 // the passes over 512 x 512 x 20 take 26, 30 and 20 us (29, 39 and 23 before), the call 92 -> 78 us,
-// 1024 x 512 x 10 101 -> 81, 256 x 256 x 80 76 -> 63. T = 64 where larger blocks would be fewer than two
-// per SM (1024 x 512 x 1: 43 -> 32 us).
+// 1024 x 512 x 10 101 -> 81, 256 x 256 x 80 76 -> 63 (launch_lines: the threads of a block).
 template <int SIGN>
 __device__ __forceinline__ void dft32(Win& v) {
   PDFT<16, SIGN>::template run<1, 0>(v.re, v.im);
@@ -378,7 +377,7 @@ __global__ void twiddle_kernel(float2* tw, int n, uint32_t* cols = nullptr) {
 // copied into unshifted order instead.
 //
 // A block forms MASK_ROWS rows of 256 columns and reports once which of them pass something: with a report
-// per element, a caller's mask that is zero nowhere took 1024 x 1024 x 1 with its passes 82 us, here 58 (49 before there were reports).
+// per element, a caller's mask that is zero nowhere took 1024 x 1024 x 1 with its passes 82 us, here 49 (22 of them the passes).
 constexpr int MASK_ROWS = 8;
 __global__ void __launch_bounds__(256) mask_kernel(float* mask, int ny, int nx, double inv_ny, double inv_nx,
                                                    float cutoff, float rolloff, const float* given, uint32_t* cols) {
@@ -455,11 +454,22 @@ cudaError_t launch_lines(const PassArgs& A, cudaStream_t st) {
   return cudaGetLastError();
 }
 
+// Threads of a block: T where that fills the GPU, 64 where it would leave SMs without a block: below two
+// blocks per SM, or one and a half for lines of 256 and 512 points that do not lie together (256 x 256 x 16
+// 17.8 -> 17.0 us; k = 1 loses: 2048 x 512 x 1 22.7 -> 24.3). Lines of 512 points and more in pass Y are the
+// exception: they are nx k elements apart, so a block of KB lines reads pieces of 8 KB bytes, and below 64
+// bytes that costs more than idle SMs (64 threads, the three passes: 1024 x 1024 x 1 27.4 us, here 22.1; x 2
+// 41.6, 28.3; 1024 x 512 x 4 39.1, 27.6; 512 x 512 x 4 22.0, 18.8), where shorter lines lose by it (256 x 256 x 1
+// 15.0, 15.4). 1024 points take 128 threads in every pass: as fast as 64 or faster in X and X'.
 template <int N, int MODE>
 cudaError_t launch_lines(const PassArgs& A, cudaStream_t st) {
   constexpr int T = N < 1024 ? 128 : 256;
   const long long blocks = (A.L.count + LineFft<N, T>::KB - 1) / LineFft<N, T>::KB;
-  return blocks < 2 * kSMs ? launch_lines<N, 64, MODE>(A, st) : launch_lines<N, T, MODE>(A, st);
+  if constexpr (N == 512 && MODE == 1)
+    return A.L.count >= 1536 && blocks < 2 * kSMs ? launch_lines<N, 256, MODE>(A, st) : launch_lines<N, T, MODE>(A, st);
+  const bool apart = (N == 256 || N == 512) && A.L.E > 1;
+  if (blocks >= (apart ? kSMs * 3 / 2 : kSMs * 2)) return launch_lines<N, T, MODE>(A, st);
+  return launch_lines<N, N == 1024 ? 128 : 64, MODE>(A, st);
 }
 
 template <int MODE>
