@@ -1009,16 +1009,31 @@ struct LPlan {
   int n_rows, single_tilt, same_prop, before, after, inside_grad, step_tilts;
   int pos_prop;   // per-position propagator tables (per-position inside tilts that apply)
   // the multislice part runs on the fused kernel's halves (var_forward, var_adjoint): 64- and 128-px
-  // windows, FP32 transforms, and not a propagator per position and step. A wave then stays in its
-  // block's registers from the first slice to the last, where a kernel per slice and step reads and
-  // writes every window: 128 px, 144 positions, 2 modes, 10 slices, a tilt per position 3.50 -> 1.79 ms;
-  // 64 px, 135 positions, 3 modes, 6 slices in near field 0.67 -> 0.53 ms. A propagator per position
+  // windows, FP32 transforms, enough slices (fused_slices), and not a propagator per position and step. A
+  // wave then stays in its block's registers from the first slice to the last, where a kernel per slice and
+  // step reads and writes every window: 128 px, 144 positions, 2 modes, 10 slices, a tilt per position 3.50 ->
+  // 1.79 ms; 64 px, 135 positions, 3 modes, 6 slices in near field 0.67 -> 0.53 ms. A propagator per position
   // and step would be a table of Bb * (Z - 1) windows, and a window of 256 px takes a cluster.
   int fused;
   int sgroups;      // scatter runs per tile
   size_t o_scpart, o_done, o_tilt_part, o_tilt_w, o_err;
   size_t o_tilts, o_tgrid, o_spec, o_fexit, o_exitb, o_pbt, o_pft, o_tpart, o_pprop, o_pprop_edge;
 };
+
+// Slices from which on the variants' multislice part gains by the fused kernel's halves. They save the
+// passes of the steps, and cost four reorderings of the waves' windows, a gradient window per probe mode
+// and, with several object modes, clusters. A kernel per slice and step / the halves, us, near field: 64 px,
+// 60 positions, 3 modes, 1 slice 263 / 279, 2 slices 302 / 292; 4 x 2 modes, 2 slices 371 / 424, 3 439 / 447,
+// 5 566 / 530; 128 px, 40 positions, 3 modes, 1 slice 367 / 391, 3 464 / 452; 2 x 2 modes, 2 slices 502 / 584,
+// 4 1.01 times, 4 x 2 modes 5 0.97 and 6 1.02 times; the inside-tilt gradient keeps a spectrum per step
+// either way and breaks even one or two slices earlier. Few modes in a batch of 120 positions or more gain a
+// slice earlier too, by the scatter in runs (64 px, 150 positions, 1 mode, 1 slice 266 / 257).
+inline int fused_slices(const LPlan& q) {
+  const int few = q.Bb >= 120 && (q.W == 64 ? q.Mp * q.Mo <= 2 : q.Mp == 1) ? 1 : 0;
+  if (q.Mo == 1) return 2 - few;
+  if (q.W == 64) return 3 - few;
+  return q.Mp <= 2 ? (q.inside_grad ? 3 : 4 - few) : (q.inside_grad ? 4 : 6);
+}
 
 inline LPlan make_lplan(const pty_problem_t* p, int engine, const pty_variant_t* v = nullptr) {
   LPlan q{};
@@ -1118,7 +1133,7 @@ inline LPlan make_lplan(const pty_problem_t* p, int engine, const pty_variant_t*
     q.pos_prop = !q.same_prop || (q.per_step && !q.single_tilt);
     q.o_pprop = take(q.pos_prop ? (size_t)q.Bb * WWs * c8 : 0);
     q.o_pprop_edge = take(q.pos_prop && edge ? (size_t)q.Bb * WWs * c8 : 0);
-    q.fused = engine == PTY_DFT_FP32_FFT && q.W <= 128 && !(q.pos_prop && q.per_step);
+    q.fused = engine == PTY_DFT_FP32_FFT && q.W <= 128 && !(q.pos_prop && q.per_step) && q.Z >= fused_slices(q);
   }
   // gradient windows: the fused halves leave one contribution per probe mode in the place of its wave
   q.o_dob = q.fused ? q.o_stack : take(nobw * WWs * c8);
