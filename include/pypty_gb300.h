@@ -127,9 +127,10 @@ int pty_simulate_patterns(const pty_problem_t* problem, const void* obj, const v
  * The same computation as pty_loss_and_direction split into its two halves, for autograd
  * and for callers that want the loss before deciding on a gradient. pty_forward runs the
  * forward multislice and the loss for every position of the sequence (compute_batch is
- * ignored: one batch) and keeps the wave stack and dL/d(exit wave) in the workspace;
- * pty_backward, called later on the same stream with the same problem and the same
- * untouched workspace, runs the adjoint and writes the gradients (and loss_sse again).
+ * ignored: one batch) and keeps the wave stack, the far-field waves and dL/dI in the
+ * workspace; pty_backward, called later on the same stream with the same problem and the
+ * same untouched workspace, runs the adjoint and writes the gradients (and loss_sse again).
+ * loss_weight scales the gradients in pty_backward; both report the weighted loss.
  * No counterpart in the reference, which always computes both (pypty/objective.py:47).
  * The workspace size is pty_split_workspace_bytes (it holds every position at once).
  */

@@ -300,7 +300,7 @@ __global__ void __launch_bounds__(512, 1) layered_fwd256_kernel(const float2* __
 // The kernel is compiled twice: PH = 1 runs the forward stages and the loss and leaves dL/dI
 // in dldi; PH = 2 starts from dldi and runs the adjoint stages. Each instance carries only
 // its own stages' code and live state (the one-kernel state machine spilled ~400 B per
-// thread; the two instances spill 208 and 76 B). Propagation steps fold the forward cross
+// thread; the instances spill 76 and 208 B). Propagation steps fold the forward cross
 // butterfly, the propagator and the inverse cross butterfly into one cluster exchange
 // (WinFFT256::cross_propagate). The next step's O_z comes by asynchronous copies into the warp's part
 // of the exchange buffer under the inverse transform's last round (plain loads: 81.2 -> 79.8 ms for 280

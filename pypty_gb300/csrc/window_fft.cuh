@@ -186,7 +186,9 @@ struct Geo {
   static constexpr int TW1 = A * 32;       // round-1 twiddle table size
   static constexpr int TW2 = W;            // round-2 twiddle table size
   static constexpr int XBUF = W * W;       // exchange buffer (float2)
-  static constexpr int MINB = W == 64 ? 4 : 1;   // resident blocks per SM the kernels aim for
+  // minimum blocks per SM of the kernels' launch bounds: at 64 px a cap of 128 registers a thread (four
+  // blocks of the FFT passes fit; the fused kernel's shared memory lets three in)
+  static constexpr int MINB = W == 64 ? 4 : 1;
 
   // real layout: element i of thread t is pixel (y, x)
   static __device__ __forceinline__ int ry(int t) { return Bq * ((t % 32) / A) + t / 32; }

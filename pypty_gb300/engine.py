@@ -378,7 +378,7 @@ class Engine:
     def forward(self, problem: _lib.Problem, obj: torch.Tensor, probe: torch.Tensor, geo: Geometry,
                 measured: torch.Tensor, stream=None):
         """Forward half (pty_forward): returns (loss_sse, workspace). The workspace holds the
-        wave stack and dL/d(exit wave) of every position until `backward` consumes it."""
+        wave stack, the far-field waves and dL/dI of every position for `backward`."""
         stream = stream or torch.cuda.current_stream(self.device)
         self._check_inputs(problem, obj, probe, measured)
         ws = torch.empty(max(_lib.split_workspace_bytes(problem), 256), dtype=torch.uint8, device=self.device)
